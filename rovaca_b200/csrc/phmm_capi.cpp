@@ -165,7 +165,9 @@ phmm_status phmm_resident_create(phmm_engine* engine, const phmm_batch* batch, i
     r->flags = want_flags != 0;
     std::string err;
     const phmm::TileTable tiles = r->eng->tiles();
-    phmm_status st = phmm::build_plan(*batch, phmm::Engine::limits_with(tiles), r->plan, err);
+    phmm::BatchScan sc;
+    phmm_status st = phmm::scan_batch(*batch, phmm::Engine::limits_with(tiles), sc, err);
+    if (st == PHMM_OK) st = phmm::build_plan(*batch, r->eng->limits_for(tiles, sc), r->plan, err);
     if (st == PHMM_OK) st = r->eng->make_slot(1000, &r->slot, err);
     if (st == PHMM_OK && (cudaEventCreate(&r->e0) != cudaSuccess || cudaEventCreate(&r->e1) != cudaSuccess)) {
         err = "event creation failed";

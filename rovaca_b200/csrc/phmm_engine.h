@@ -26,6 +26,9 @@ struct Capacity {
     uint64_t events = 0, hap_allele = 0, allele_lk = 0, gl = 0;
     bool covers(const Capacity& o) const;
     Capacity grown_to(const Capacity& need) const;
+    // room for batches a little larger: work items and bases vary from batch to batch of one shape,
+    // and growing an arena costs up to half a second (allocation, graph capture)
+    Capacity with_slack() const;
     static Capacity max_of(const Capacity& a, const Capacity& b);
 };
 
@@ -133,6 +136,8 @@ public:
         l.tiles = &t;
         return l;
     }
+    // The same with the work-item streams sized for a batch of these sizes on this device.
+    PlanLimits limits_for(const TileTable& t, const BatchScan& sc) const;
     // Runs an uploaded plan once with every class alone on the slot's main stream, timing each
     // launch with CUDA events (class_ms[kNumClasses], 0 where a class has no work).
     phmm_status profile_classes(Slot& s, const Plan& plan, float* class_ms, std::string& err);
@@ -162,6 +167,7 @@ public:
 
 private:
     Engine() = default;
+    bool use_graph(const Plan& plan) const;  // replay the captured graph for this batch
     phmm_status ensure_capacity(Slot& s, const Plan& plan, std::string& err);
     phmm_status launch_pipeline(Slot& s, bool want_flags, const Plan* plan, const TileTable& tiles, std::string& err);
     phmm_status capture_graph(Slot& s, bool want_flags, const TileTable& tiles, std::string& err);

@@ -12,6 +12,7 @@
 #include "phmm_plan.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <thread>
 
@@ -91,6 +92,19 @@ bool TileTable::valid(std::string& err) const
     return true;
 }
 
+// kRunSetupCols: an item's fill and drain (31 columns) and its row set-up, in columns' time.  Measured
+// on B200 (one call end to end, milliseconds; runs of up to 8192 columns first, then 24, 96, 160): one
+// region of 16 haplotypes and 250 reads 1.16, 0.41, 0.42, 0.40; 8 regions 3.13, 0.94, 0.97, 0.95; 150
+// regions with per-base gaps 23.8, 21.5, 21.2, 21.5; 24 regions of long reads 21.0, 15.3, 15.1, 15.3;
+// 1,000 regions 104.8, 104.6, 104.9, 104.9; 60 low-quality regions 39.8, 39.9, 39.4, 39.4.
+constexpr double kRunSetupCols = 96.0;
+
+uint32_t run_cols_for(uint64_t stream_cols, uint64_t warps)
+{
+    const double c = std::sqrt((double)stream_cols * kRunSetupCols / (double)std::max<uint64_t>(warps, 1));
+    return (uint32_t)std::min<double>(std::max(c, 1.0), PlanLimits().max_stream_single);
+}
+
 phmm_status scan_batch(const phmm_batch& b, const PlanLimits& lim, BatchScan& s, std::string& err)
 {
     s = BatchScan();
@@ -120,7 +134,7 @@ phmm_status scan_batch(const phmm_batch& b, const PlanLimits& lim, BatchScan& s,
     // offsets non-decreasing, lengths within the limits; per region the non-empty pairs and cells
     uint64_t h = 0, r = 0;
     for (uint32_t g = 0; g < b.n_regions; ++g) {
-        uint64_t hcols = 0, hnon = 0, rrows = 0, rnon = 0;
+        uint64_t hcols = 0, hnon = 0, rrows = 0, rnon = 0, rstripes = 0;
         for (uint32_t k = 0; k < b.n_haps[g]; ++k, ++h) {
             if (b.hap_off[h + 1] < b.hap_off[h]) {
                 err = "hap_off is not non-decreasing at " + std::to_string(h + 1);
@@ -146,10 +160,12 @@ phmm_status scan_batch(const phmm_batch& b, const PlanLimits& lim, BatchScan& s,
             }
             rrows += R;
             rnon += R > 0;
+            rstripes += (R + (uint64_t)kWarp * kMaxK - 1) / ((uint64_t)kWarp * kMaxK);
         }
         s.out_total += (uint64_t)b.n_haps[g] * b.n_reads[g];
         s.pairs += hnon * rnon;
         s.cells += hcols * rrows;
+        s.stream_cols += hcols * ((rstripes + 1) / 2);
     }
     s.hap_bases = b.hap_off[nh] - s.hap_base0;
     s.read_bases = b.read_off[nr] - s.read_base0;

@@ -76,7 +76,18 @@ struct BatchScan {
     uint64_t hap_base0 = 0, read_base0 = 0;  // hap_off[0], read_off[0]
     uint64_t hap_bases = 0, read_bases = 0, out_total = 0;
     uint64_t pairs = 0, cells = 0;           // pairs with a non-empty read and haplotype, their cells
+    // columns a warp streams over the whole batch: per region its haplotype bases times half its
+    // reads (two reads a warp), a read counting once per 256 rows
+    uint64_t stream_cols = 0;
 };
+
+// The longest haplotype stream of a work item for a batch that streams `stream_cols` columns over
+// `warps` resident warps (single-stripe items; multi-stripe items take half).  A long run pays the
+// fill, drain and row set-up of an item once for many haplotypes; a short one leaves a small batch
+// more items than warps, and a large one a shorter last wave.  With o columns' worth of set-up per
+// item the pass takes about (stream_cols (1 + o / c) / warps + c) steps, least at
+// c = sqrt(stream_cols o / warps).
+uint32_t run_cols_for(uint64_t stream_cols, uint64_t warps);
 
 // Validation shared by every entry point: counts, non-decreasing offsets, the reference limits and
 // the pointers the batch needs.  Returns PHMM_OK, PHMM_ERR_INVALID_ARGUMENT or

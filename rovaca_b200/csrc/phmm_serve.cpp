@@ -385,7 +385,14 @@ void Server::worker(int idx)
             const TileTable tiles = eng->tiles();
             PlanLimits lim = Engine::limits_with(tiles);
             if (api) lim.region_api = params.data();
-            st = build_plan(b, lim, plan, berr);
+            BatchScan sc;
+            st = scan_batch(b, lim, sc, berr);
+            if (st == PHMM_OK) {
+                const PlanLimits sized = eng->limits_for(tiles, sc);
+                lim.max_stream_single = sized.max_stream_single;
+                lim.max_stream_multi = sized.max_stream_multi;
+                st = build_plan(b, lim, plan, berr);
+            }
             if (st == PHMM_OK && n_events) {
                 // events of the batch, in request order
                 uint64_t gl_o = 0, alk_o = 0;

@@ -64,6 +64,21 @@ def test_graph_and_direct_launch_agree(engine, engine_direct, ref_regions):
         assert np.array_equal(fa, fb)
 
 
+@pytest.mark.parametrize("regions", [1, 7, 90])
+def test_work_item_runs_and_launch_form_do_not_change_results(engine, engine_direct, regions):
+    """The haplotype runs of the work items are sized to the batch, and a batch of 2e10 cells or more
+    (the 90 regions here) replays the captured graph where smaller ones launch directly: the same
+    bits and flags as every region on its own without graphs."""
+    pb = synth.config1(regions, seed=21)
+    got, flags, st = engine.compute(pb, want_flags=True)
+    assert (st["cells"] >= 2e10) == (regions == 90)
+    offs = pb.out_offsets()
+    for g in sorted({0, regions // 2, regions - 1}):
+        a, f, _ = engine_direct.compute(pb.subset([g]), want_flags=True)
+        assert np.array_equal(got[offs[g]:offs[g + 1]], a, equal_nan=True)
+        assert np.array_equal(flags[offs[g]:offs[g + 1]], f)
+
+
 def test_region_result_independent_of_batch(engine):
     """Per-pair arithmetic does not depend on what else is in the batch."""
     pb = synth.config1(12, seed=5)
