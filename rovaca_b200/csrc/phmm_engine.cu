@@ -408,10 +408,16 @@ phmm_status Engine::realign_enqueue(Slot& s, RealignBatch& rb, std::string& err)
     b.compact = (uint32_t*)(d + rb.o_compact);
     b.scratch = (uint8_t*)(d + rb.o_scratch);
     const SwParams prm{10, -15, -30, -5};  // sw_parameters_genotype, lib/sw_avx/sw_avx.c:15
-    st = sw_launch(rb.plan, prm, 0, b, s.main, nullptr, nullptr, nullptr, err);
+    // the class streams of the pipeline are idle again (s.main has joined them)
+    static_assert(kSwGroups <= kNumClasses, "one class stream per group");
+    SwFork fork;
+    fork.side = s.side;
+    fork.done = s.ev_side;
+    fork.fork = s.ev_fork;
+    st = sw_launch(rb.plan, prm, 0, b, s.main, &fork, nullptr, nullptr, nullptr, err);
     if (st != PHMM_OK) return st;
     s.launches += 1 + 2;
-    for (int c = 0; c < kSwClasses; ++c) s.launches += rb.plan.grid[c] ? 1 : 0;
+    for (int g = 0; g < kSwGroups; ++g) s.launches += rb.plan.grid[g] ? 1 : 0;
     // total, results and best haplotypes come back with the rest of the batch's outputs
     PHMM_CK(cudaMemcpyAsync(h, d + rb.o_total, rb.head_bytes(), cudaMemcpyDeviceToHost, s.main));
     return PHMM_OK;

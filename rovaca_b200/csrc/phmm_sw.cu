@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "phmm_sw.h"
+#include "phmm_sw16.cuh"
 #include "phmm_types.h"
 
 namespace phmm {
@@ -46,23 +47,6 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kStIns = 1, kStDel = 2, kStInsExt = 4, kStDelExt = 8, kStClip = 9;
-
-struct SwView {
-    const SwItem* items;
-    const uint32_t* order;       // this class's item indices, most cells first
-    uint32_t n;
-    const uint8_t* hap;
-    const uint8_t* read;
-    SwParams prm;
-    int variant;
-    uint8_t* scratch;
-    uint64_t stride;             // scratch bytes per warp
-    unsigned int* claim;
-    phmm_sw_result* out;
-    const uint64_t* slot_off;    // per item: its CIGAR slot in `ops` (min(cap, nrow + ncol) ops)
-    uint32_t* ops;
-    uint32_t cigar_cap;
-};
 
 // Score add: two's-complement 32-bit, wrapped to 16 bits in the wrap-around class when the
 // alignment runs the int16 kernel (w16; an int32 alignment in that class adds in 32 bits).
@@ -159,7 +143,7 @@ __device__ void sw_one(const SwView& v, uint32_t idx, int lane, uint8_t* scr, ui
             if (s > 0 && lane == 0) { bnh = bh[1]; bne = be[1]; }
             int hprev = 0;                         // H(i-1, left column) of this lane
             int hout = 0, eout = low;              // H, E of this lane's last column, previous step
-            uint32_t* bts = bt + (uint64_t)s * nrow * ROW;
+            uint32_t* bts = bt + (uint64_t)s * (nrow + 31) * ROW;
             const int steps = nrow + 31;
             // one wavefront step; FULL: every lane is on a real row (steps 31 .. nrow - 1), so the
             // activity tests drop out of the cell loop
@@ -204,7 +188,7 @@ __device__ void sw_one(const SwView& v, uint32_t idx, int lane, uint8_t* scr, ui
                 hout = act ? hl : 0;               // a lane before its first row stands for row 0
                 eout = act ? el : low;
                 if (act) {
-                    uint32_t* row = bts + (uint64_t)(i - 1) * ROW + lane;
+                    uint32_t* row = bts + (uint64_t)t * ROW + lane;  // one row per step: contiguous
 #pragma unroll
                     for (int w = 0; w < NW; ++w) row[w * 32] = code[w];
                     if (i == nrow) {
@@ -274,17 +258,18 @@ __device__ void sw_one(const SwView& v, uint32_t idx, int lane, uint8_t* scr, ui
     int bs = -1, br0 = 0, br1 = -1;
     while (i > 0 && j > 0) {
         const int s = (j - 1) / S, jj = (j - 1) - s * S, ln = jj / K, k = jj - ln * K;
-        if (s != bs || i - 1 < br0 || i - 1 > br1) {
+        const int tt = i - 1 + ln;  // the step at which lane ln was on row i
+        if (s != bs || tt < br0 || tt > br1) {
             bs = s;
-            br1 = i - 1;
+            br1 = tt;
             br0 = max(0, br1 - BAND_ROWS + 1);
-            const uint32_t* src = bt + ((uint64_t)s * nrow + br0) * ROW;
+            const uint32_t* src = bt + ((uint64_t)s * (nrow + 31) + br0) * ROW;
             const int words = (br1 - br0 + 1) * ROW;
             __syncwarp();
             for (int q = lane; q < words; q += 32) band[q] = src[q];
             __syncwarp();
         }
-        const uint32_t w = band[(i - 1 - br0) * ROW + (k >> 3) * 32 + ln];
+        const uint32_t w = band[(tt - br0) * ROW + (k >> 3) * 32 + ln];
         const int b = (int)((w >> (4 * (k & 7))) & 15u);
         if (state == kStInsExt) {
             --j;
@@ -351,6 +336,24 @@ __global__ void __launch_bounds__(32 * kSwBlockWarps, sw_min_blocks<K>()) sw_ker
             sw_one<K, WRAP, true>(v, idx, lane, scr, band[wib]);
         else
             sw_one<K, WRAP, false>(v, idx, lane, scr, band[wib]);
+    }
+}
+
+// Two alignments per warp (phmm_sw16.cuh): one-warp blocks, each claiming pairs of neighbours in the
+// launch's order (longest haplotype first, so that the two are of about one length).
+template <int K>
+__global__ void __launch_bounds__(32, K <= 12 ? 16 : 12) sw16_kernel(SwView v, uint32_t max_rows)
+{
+    extern __shared__ uint4 sw16_shared[];
+    const int lane = threadIdx.x;
+    uint8_t* scr = v.scratch + (uint64_t)blockIdx.x * v.stride;
+    for (;;) {
+        unsigned int p = 0;
+        if (lane == 0) p = atomicAdd(v.claim, 1u);
+        p = __shfl_sync(kFull, p, 0);
+        if (2 * p >= v.n) break;
+        sw16_pair<K>(v, v.order[2 * p], 2 * p + 1 < v.n ? v.order[2 * p + 1] : 0xffffffffu, lane, scr, (char*)sw16_shared,
+                     max_rows);
     }
 }
 
@@ -517,6 +520,30 @@ __global__ void __launch_bounds__(kRealignThreads) realign_items_kernel(RealignV
     }
 }
 
+using Sw16Kernel = void (*)(SwView, uint32_t);
+const Sw16Kernel kSw16Kernels[kSwWrapClass] = {
+    sw16_kernel<1>, sw16_kernel<2>, sw16_kernel<3>,  sw16_kernel<4>,  sw16_kernel<5>,  sw16_kernel<6>,  sw16_kernel<7>,
+    sw16_kernel<8>, sw16_kernel<10>, sw16_kernel<12>, sw16_kernel<16>, sw16_kernel<20>, sw16_kernel<24>,
+};
+uint32_t sw16_shared_bytes(int c, uint32_t max_rows)
+{
+    switch (kSwK[c]) {
+    case 1: return Sw16Shared<1>::bytes(max_rows);
+    case 2: return Sw16Shared<2>::bytes(max_rows);
+    case 3: return Sw16Shared<3>::bytes(max_rows);
+    case 4: return Sw16Shared<4>::bytes(max_rows);
+    case 5: return Sw16Shared<5>::bytes(max_rows);
+    case 6: return Sw16Shared<6>::bytes(max_rows);
+    case 7: return Sw16Shared<7>::bytes(max_rows);
+    case 8: return Sw16Shared<8>::bytes(max_rows);
+    case 10: return Sw16Shared<10>::bytes(max_rows);
+    case 12: return Sw16Shared<12>::bytes(max_rows);
+    case 16: return Sw16Shared<16>::bytes(max_rows);
+    case 20: return Sw16Shared<20>::bytes(max_rows);
+    default: return Sw16Shared<24>::bytes(max_rows);
+    }
+}
+
 using SwKernel = void (*)(SwView);
 
 const SwKernel kSwKernels[kSwClasses] = {
@@ -556,7 +583,7 @@ struct SwArenaLayout {
         hap = a(slot_off + 8ull * n);
         read = a(hap + std::max<uint64_t>(hap_bytes, 1));
         claim = a(read + std::max<uint64_t>(read_bytes, 1));
-        total = a(claim + 4ull * kSwClasses);
+        total = a(claim + 4ull * kSwGroups);
         out = total + 8;
         slots = a(out + sizeof(phmm_sw_result) * (uint64_t)n);
         compact = a(slots + 4ull * std::max<uint64_t>(nslots, 1));
@@ -666,6 +693,9 @@ phmm_status device_info(int device, SwDeviceInfo& out, std::string& err)
             SW_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kSwKernels[c], 32 * kSwBlockWarps, 0));
             di.occ[c] = std::max(b, 1);
         }
+        for (int c = 0; c < kSwWrapClass; ++c)
+            SW_CK(cudaFuncSetAttribute(kSw16Kernels[c], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sw16_shared_bytes(c, kSwMaxSeq - 1)));
         SW_CK(cudaSetDevice(cur));
         di.ready = true;
     }
@@ -684,12 +714,16 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
     p = SwPlan();
     p.n = n;
     p.cigar_cap = std::min<uint32_t>(cigar_cap, kSwMaxSeq - 1);
-    std::vector<uint8_t> cls(n);
-    uint32_t counts[kSwClasses] = {};
+    std::vector<uint8_t> grp(n);
+    uint32_t counts[kSwGroups] = {};
     p.slot_off.resize(n);
     for (uint32_t q = 0; q < n; ++q) {
-        cls[q] = (uint8_t)sw_class_of(prm, variant, nrow[q], ncol[q]);
-        ++counts[cls[q]];
+        const int c = sw_class_of(prm, variant, nrow[q], ncol[q]);
+        const bool packs = c != kSwWrapClass && sw_packs(prm, nrow[q], ncol[q], kSwK[c]);
+        const int g = packs ? c : kSwWrapClass + c;
+        grp[q] = (uint8_t)g;
+        ++counts[g];
+        p.max_rows[g] = std::max(p.max_rows[g], nrow[q]);
         p.cells += (uint64_t)nrow[q] * ncol[q];
         p.slot_off[q] = p.slots;
         if (std::max(nrow[q], ncol[q]) < (uint32_t)kSwMaxSeq)  // runs <= rows + columns consumed
@@ -700,68 +734,109 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
         return PHMM_ERR_LIMIT_EXCEEDED;
     }
     p.begin[0] = 0;
-    for (int c = 0; c < kSwClasses; ++c) p.begin[c + 1] = p.begin[c] + counts[c];
-    // one counting sort: by class, then most cells first in buckets of 4096 cells (the claim order
-    // only balances the persistent warps' load, so buckets are as good as an exact order)
+    for (int g = 0; g < kSwGroups; ++g) p.begin[g + 1] = p.begin[g] + counts[g];
+    // one counting sort: by group, then longest first in buckets: two rows in the 16-bit groups, whose
+    // warps run neighbours together for the longer one's rows, 4096 cells in the others (there the
+    // order only balances the persistent warps' load)
     constexpr uint32_t kBuckets = 1024;
     auto key = [&](uint32_t q) {
-        const uint64_t b = std::min<uint64_t>(kBuckets - 1, ((uint64_t)nrow[q] * ncol[q]) >> 12);
-        return (uint32_t)cls[q] * kBuckets + (kBuckets - 1 - (uint32_t)b);
+        const uint64_t len = grp[q] < kSwWrapClass ? nrow[q] >> 1 : ((uint64_t)nrow[q] * ncol[q]) >> 12;
+        return (uint32_t)grp[q] * kBuckets + (kBuckets - 1 - (uint32_t)std::min<uint64_t>(kBuckets - 1, len));
     };
-    std::vector<uint32_t> start((size_t)kSwClasses * kBuckets + 1, 0);
+    std::vector<uint32_t> start((size_t)kSwGroups * kBuckets + 1, 0);
     for (uint32_t q = 0; q < n; ++q) ++start[key(q) + 1];
     for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
     p.order.assign(n, 0);
     for (uint32_t q = 0; q < n; ++q) p.order[start[key(q)]++] = q;
-    p.scratch = 0;
-    for (int c = 0; c < kSwClasses; ++c) {
-        auto first = p.order.begin() + p.begin[c], lastp = p.order.begin() + p.begin[c + 1];
-        uint64_t stride = 256;
-        for (auto it = first; it != lastp; ++it) {
-            if (std::max(nrow[*it], ncol[*it]) >= (uint32_t)kSwMaxSeq) continue;  // refused: no scratch
-            stride = std::max(stride, sw_layout(nrow[*it], ncol[*it], kSwK[c]).total);
+    uint64_t need[kSwGroups] = {}, sum = 0, most = 0;
+    for (int g = 0; g < kSwGroups; ++g) {
+        const uint32_t m = counts[g];
+        if (m == 0) continue;
+        const int c = sw_group_class(g);
+        uint64_t blocks, warps;
+        if (g < kSwWrapClass) {
+            int occ = 0;
+            SW_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kSw16Kernels[c], 32,
+                                                                sw16_shared_bytes(c, p.max_rows[g])));
+            p.stride[g] = std::max<uint64_t>(256, sw16_layout(p.max_rows[g], kSwK[c]).total);
+            blocks = std::min<uint64_t>(((uint64_t)m + 1) / 2, (uint64_t)std::max(occ, 1) * di.sms);
+            warps = 1;
+        } else {
+            uint64_t stride = 256;
+            for (uint32_t k = p.begin[g]; k < p.begin[g + 1]; ++k) {
+                const uint32_t q = p.order[k];
+                if (std::max(nrow[q], ncol[q]) >= (uint32_t)kSwMaxSeq) continue;  // refused: no scratch
+                stride = std::max(stride, sw_layout(nrow[q], ncol[q], kSwK[c]).total);
+            }
+            p.stride[g] = stride;
+            blocks = std::min<uint64_t>((m + kSwBlockWarps - 1) / kSwBlockWarps, (uint64_t)di.occ[c] * di.sms);
+            warps = kSwBlockWarps;
         }
-        p.stride[c] = stride;
-        const uint32_t m = counts[c];
-        uint64_t g = std::min<uint64_t>((m + kSwBlockWarps - 1) / kSwBlockWarps, (uint64_t)di.occ[c] * di.sms);
-        g = std::min<uint64_t>(g, std::max<uint64_t>(1, kSwScratchCap / (kSwBlockWarps * stride)));
-        p.grid[c] = m == 0 ? 0 : (int)g;
-        p.scratch = std::max(p.scratch, (uint64_t)p.grid[c] * kSwBlockWarps * stride);
+        blocks = std::min<uint64_t>(blocks, std::max<uint64_t>(1, kSwScratchCap / (warps * p.stride[g])));
+        p.grid[g] = (int)blocks;
+        need[g] = blocks * warps * p.stride[g];
+        sum += need[g];
+        most = std::max(most, need[g]);
+    }
+    // the groups run side by side, each in scratch of its own, when all of it fits the bound
+    p.concurrent = sum <= kSwScratchCap;
+    p.scratch = p.concurrent ? sum : most;
+    uint64_t at = 0;
+    for (int g = 0; g < kSwGroups && p.concurrent; ++g) {
+        p.scratch_off[g] = at;
+        at += need[g];
     }
     p.gather_blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((n + 7) / 8, (uint64_t)di.sms * 8));
     return PHMM_OK;
 }
 
 phmm_status sw_launch(const SwPlan& p, const SwParams& prm, int variant, const SwDeviceBufs& b, cudaStream_t st,
-                      cudaEvent_t ev0, cudaEvent_t ev1, float* class_ms, std::string& err)
+                      const SwFork* fork, cudaEvent_t ev0, cudaEvent_t ev1, float* class_ms, std::string& err)
 {
     if (p.n == 0) return PHMM_OK;
-    SW_CK(cudaMemsetAsync(b.claim, 0, sizeof(unsigned int) * kSwClasses, st));
-    for (int c = 0; c < kSwClasses; ++c) {
-        if (class_ms) class_ms[c] = 0.f;
-        if (p.grid[c] == 0) continue;
+    SW_CK(cudaMemsetAsync(b.claim, 0, sizeof(unsigned int) * kSwGroups, st));
+    int groups = 0;
+    for (int g = 0; g < kSwGroups; ++g) groups += p.grid[g] > 0;
+    const bool side = fork && p.concurrent && !class_ms && groups > 1;
+    if (class_ms)
+        for (int c = 0; c < kSwClasses; ++c) class_ms[c] = 0.f;
+    if (side) SW_CK(cudaEventRecord(fork->fork, st));
+    for (int g = 0; g < kSwGroups; ++g) {
+        if (p.grid[g] == 0) continue;
+        const int c = sw_group_class(g);
         SwView v{};
         v.items = b.items;
-        v.order = b.order + p.begin[c];
-        v.n = p.begin[c + 1] - p.begin[c];
+        v.order = b.order + p.begin[g];
+        v.n = p.begin[g + 1] - p.begin[g];
         v.hap = b.hap;
         v.read = b.read;
         v.prm = prm;
         v.variant = variant;
-        v.scratch = b.scratch;
-        v.stride = p.stride[c];
-        v.claim = b.claim + c;
+        v.scratch = b.scratch + p.scratch_off[g];
+        v.stride = p.stride[g];
+        v.claim = b.claim + g;
         v.out = b.out;
         v.slot_off = b.slot_off;
         v.ops = b.slots;
         v.cigar_cap = p.cigar_cap;
-        if (class_ms) SW_CK(cudaEventRecord(ev0, st));
-        kSwKernels[c]<<<p.grid[c], 32 * kSwBlockWarps, 0, st>>>(v);
+        const cudaStream_t s = side ? fork->side[g] : st;
+        if (side) SW_CK(cudaStreamWaitEvent(s, fork->fork, 0));
+        if (class_ms) SW_CK(cudaEventRecord(ev0, s));
+        if (g < kSwWrapClass)
+            kSw16Kernels[c]<<<p.grid[g], 32, sw16_shared_bytes(c, p.max_rows[g]), s>>>(v, p.max_rows[g]);
+        else
+            kSwKernels[c]<<<p.grid[g], 32 * kSwBlockWarps, 0, s>>>(v);
         SW_CK(cudaGetLastError());
         if (class_ms) {
-            SW_CK(cudaEventRecord(ev1, st));
+            float ms = 0.f;
+            SW_CK(cudaEventRecord(ev1, s));
             SW_CK(cudaEventSynchronize(ev1));
-            SW_CK(cudaEventElapsedTime(&class_ms[c], ev0, ev1));
+            SW_CK(cudaEventElapsedTime(&ms, ev0, ev1));
+            class_ms[c] += ms;
+        }
+        if (side) {
+            SW_CK(cudaEventRecord(fork->done[g], s));
+            SW_CK(cudaStreamWaitEvent(st, fork->done[g], 0));
         }
     }
     sw_scan_kernel<<<1, kScanThreads, 0, st>>>(b.out, p.n, p.cigar_cap, b.total);
@@ -789,7 +864,7 @@ void RealignBatch::layout()
     o_slot = a(o_order + 4ull * n);
     o_items = a(o_slot + 8ull * n);
     o_claim = a(o_items + sizeof(SwItem) * n);
-    o_total = a(o_claim + 4ull * kSwClasses);
+    o_total = a(o_claim + 4ull * kSwGroups);
     o_out = o_total + 8;
     o_best = o_out + sizeof(phmm_sw_result) * n;
     o_slots = a(o_best + 4ull * n);
@@ -819,6 +894,14 @@ phmm_status SwAligner::create(int device, SwAligner** out, std::string& err)
     SW_CKC(cudaStreamCreateWithFlags(&a->stream_, cudaStreamNonBlocking));
     SW_CKC(cudaEventCreate(&a->ev_[0]));
     SW_CKC(cudaEventCreate(&a->ev_[1]));
+    SW_CKC(cudaEventCreateWithFlags(&a->ev_fork_, cudaEventDisableTiming));
+    for (int g = 0; g < kSwGroups; ++g) {
+        SW_CKC(cudaStreamCreateWithFlags(&a->side_[g], cudaStreamNonBlocking));
+        SW_CKC(cudaEventCreateWithFlags(&a->ev_side_[g], cudaEventDisableTiming));
+    }
+    a->fork_.side = a->side_;
+    a->fork_.done = a->ev_side_;
+    a->fork_.fork = a->ev_fork_;
 #undef SW_CKC
     *out = a;
     return PHMM_OK;
@@ -831,6 +914,11 @@ SwAligner::~SwAligner()
     if (pinned_) cudaFreeHost(pinned_);
     for (auto& e : ev_)
         if (e) cudaEventDestroy(e);
+    if (ev_fork_) cudaEventDestroy(ev_fork_);
+    for (int g = 0; g < kSwGroups; ++g) {
+        if (ev_side_[g]) cudaEventDestroy(ev_side_[g]);
+        if (side_[g]) cudaStreamDestroy(side_[g]);
+    }
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -929,7 +1017,7 @@ phmm_status SwAligner::align(const SwParams& prm, int variant, uint32_t n, const
     if (read_bytes) staged_copy(h + L.read, read, read_bytes);
     SW_CK(cudaMemcpyAsync(d, h, L.in_bytes(), cudaMemcpyHostToDevice, stream_));
     SW_CK(cudaEventRecord(ev_[0], stream_));
-    st = sw_launch(p, prm, variant, L.bufs(d), stream_, ev_[0], ev_[1], nullptr, err);
+    st = sw_launch(p, prm, variant, L.bufs(d), stream_, &fork_, nullptr, nullptr, nullptr, err);
     if (st != PHMM_OK) return st;
     SW_CK(cudaEventRecord(ev_[1], stream_));
     st = read_back(d, L, n, out, cigars, cigar_capacity, cigar_total, err);
@@ -993,7 +1081,7 @@ phmm_status SwAligner::resident_run(Resident* r, int iterations, float* ms_per_r
     if (iterations > 0) {
         SW_CK(cudaEventRecord(ev_[0], stream_));
         for (int it = 0; it < iterations; ++it) {
-            phmm_status st = sw_launch(r->plan, r->prm, r->variant, b, stream_, nullptr, nullptr, nullptr, err);
+            phmm_status st = sw_launch(r->plan, r->prm, r->variant, b, stream_, &fork_, nullptr, nullptr, nullptr, err);
             if (st != PHMM_OK) return st;
         }
         SW_CK(cudaEventRecord(ev_[1], stream_));
@@ -1003,7 +1091,7 @@ phmm_status SwAligner::resident_run(Resident* r, int iterations, float* ms_per_r
         if (ms_per_run) *ms_per_run = ms / iterations;
     }
     if (class_ms) {
-        phmm_status st = sw_launch(r->plan, r->prm, r->variant, b, stream_, ev_[0], ev_[1], class_ms, err);
+        phmm_status st = sw_launch(r->plan, r->prm, r->variant, b, stream_, nullptr, ev_[0], ev_[1], class_ms, err);
         if (st != PHMM_OK) return st;
         SW_CK(cudaStreamSynchronize(stream_));
     }

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/phmm_b200.h"
+#include "phmm_types.h"
 
 namespace phmm {
 
@@ -31,9 +32,32 @@ constexpr int kSwBandWords = 1024;   // trace-back band in shared memory per war
 constexpr int kSwClasses = 14;       // 13 stripe widths (kSwK) + the 16-bit wrap-around class
 constexpr int kSwWrapClass = 13;
 constexpr int kSwK[kSwClasses] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16, 20, 24, 24};
+// Kernel launches of a batch: the 13 stripe widths with two alignments per warp in 16-bit halves
+// (phmm_sw16.cuh), then the 14 classes with one alignment per warp.
+constexpr int kSwGroups = kSwWrapClass + kSwClasses;
+PHMM_HD inline int sw_group_class(int g) { return g < kSwWrapClass ? g : g - kSwWrapClass; }
+
+// What one class launch works on.
+struct SwView {
+    const SwItem* items;
+    const uint32_t* order;       // this launch's item indices
+    uint32_t n;
+    const uint8_t* hap;
+    const uint8_t* read;
+    SwParams prm;
+    int variant;
+    uint8_t* scratch;
+    uint64_t stride;             // scratch bytes per warp
+    unsigned int* claim;
+    phmm_sw_result* out;
+    const uint64_t* slot_off;    // per item: its CIGAR slot in `ops` (min(cap, nrow + ncol) ops)
+    uint32_t* ops;
+    uint32_t cigar_cap;
+};
 
 // Per-warp scratch layout of one alignment (bytes, 256-aligned sections):
-//   bt    [stripes][nrow][32 * nw] u32: per cell a 4-bit code (state 1/2 | extension flags 4/8)
+//   bt    [stripes][nrow + 31][32 * nw] u32: per cell a 4-bit code (state 1/2 | extension flags 4/8),
+//         one row per wavefront step
 //   bh/be [nrow + 1] i32: H and E of the stripe's right edge column, handed to the next stripe
 //   lrow  [ncol + 1] i32: H of the last row; lcol [nrow + 1] i32: H of the last column
 //   runs  [nrow + ncol + 4] u32: CIGAR runs in trace-back order
@@ -50,7 +74,7 @@ __host__ __device__ inline SwLayout sw_layout(uint32_t nrow, uint32_t ncol, int 
     const uint64_t stripes = ncol ? (ncol + cols - 1) / cols : 1;
     SwLayout L;
     L.bt = 0;
-    uint64_t o = sw_align256(stripes * nrow * 32ull * nw * 4ull);
+    uint64_t o = sw_align256(stripes * (nrow + 31ull) * 32ull * nw * 4ull);
     L.bh = o;
     o = sw_align256(o + 4ull * (nrow + 1));
     L.be = o;
@@ -88,26 +112,50 @@ __host__ __device__ inline bool sw_w16_cannot_wrap(int32_t match, int32_t mismat
            ext >= -16384 && (match <= 0 || (long long)min_len * match <= 32767);
 }
 
+// The 16-bit form of stripe width K: stored scores are biased by this much, so that every quantity of
+// the recurrences is at least 0.  E(i,j) >= open + (j - 1) ext and H >= E; one more opening, extension
+// or mismatch is added to them.
+PHMM_HD inline int sw16_bias(const SwParams& p, int K)
+{
+    return -(2 * p.gap_open + p.mismatch + (32 * K + 2) * p.gap_extend) + 16;
+}
+// Whether alignments of at most 32 * K read bases run two per warp in 16-bit halves: parameters for
+// which pad columns stand for the boundary (gap_open <= 0, gap_extend < 0, mismatch <= 0 <= match), a
+// bias under 8,000 (E then stays above the reference's 16-bit cutoff of -8192, which can change
+// nothing, see sw_cutoff_can_bind) and scores that fit 15 bits with it.
+inline bool sw_packs(const SwParams& p, uint32_t nrow, uint32_t ncol, int K)
+{
+    if (ncol > 32u * (uint32_t)K || nrow >= (uint32_t)kSwMaxSeq) return false;
+    if (p.gap_open > 0 || p.gap_open < -4000 || p.gap_extend >= 0 || p.gap_extend < -4000 || p.mismatch > 0 ||
+        p.mismatch < -8000 || p.match < 0 || p.match > 32000)
+        return false;
+    const int bias = sw16_bias(p, K);
+    return bias < 8000 && bias + (32 * K + 1) * (long long)p.match <= 32000;
+}
+
 int sw_class_of(const SwParams& prm, int variant, uint32_t nrow, uint32_t ncol);
 
-// Host plan of one batch of alignments: kernel class of each (by read columns, or the wrap-around
-// class), alignments grouped by class most cells first, CIGAR slots, grids and scratch.
+// Host plan of one batch of alignments: launch group of each (by read columns and parameters),
+// alignments ordered by group, longest first, CIGAR slots, grids and scratch.
 struct SwPlan {
     uint32_t n = 0;
     uint32_t cigar_cap = 0;
-    std::vector<uint32_t> order;             // item indices grouped by class, most cells first
+    std::vector<uint32_t> order;             // item indices by group, longest first
     std::vector<uint64_t> slot_off;          // per item: its CIGAR slot (ops) in the slot buffer
     uint64_t slots = 0;                      // ops of all slots
-    uint32_t begin[kSwClasses + 1] = {};
-    uint64_t stride[kSwClasses] = {};        // scratch bytes per warp of each class
-    int grid[kSwClasses] = {};
+    uint32_t begin[kSwGroups + 1] = {};
+    uint64_t stride[kSwGroups] = {};         // scratch bytes per warp of each group
+    uint64_t scratch_off[kSwGroups] = {};    // its scratch
+    uint32_t max_rows[kSwGroups] = {};       // longest haplotype of the group (16-bit groups)
+    int grid[kSwGroups] = {};
+    bool concurrent = true;                  // the groups have disjoint scratch and may run together
     int gather_blocks = 1;
-    uint64_t scratch = 0;                    // bytes for the largest class launch
+    uint64_t scratch = 0;                    // bytes of all of it
     uint64_t cells = 0;
 };
 
 // Device buffers of one batch (see SwPlan for their sizes: n items, n results, `slots` ops twice,
-// `scratch` bytes, kSwClasses claim counters).
+// `scratch` bytes, kSwGroups claim counters).
 struct SwDeviceBufs {
     const SwItem* items = nullptr;
     const uint32_t* order = nullptr;
@@ -126,10 +174,18 @@ struct SwDeviceBufs {
 // columns (read lengths).
 phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, const uint32_t* nrow,
                     const uint32_t* ncol, uint32_t cigar_cap, SwPlan& p, std::string& err);
-// Launches a planned batch on stream st: the class kernels, the CIGAR offset scan and the gather.
+// Streams and events (kSwGroups of each, and one more event) for the groups of a batch to run side by
+// side; the caller's stream waits for all of them.
+struct SwFork {
+    cudaStream_t* side = nullptr;
+    cudaEvent_t* done = nullptr;
+    cudaEvent_t fork = nullptr;
+};
+// Launches a planned batch on stream st: the group kernels (side by side on the fork's streams when the
+// plan allows it and `fork` is given), the CIGAR offset scan and the gather.
 // class_ms (optional, kSwClasses): every class timed alone with ev0/ev1 (synchronising).
 phmm_status sw_launch(const SwPlan& p, const SwParams& prm, int variant, const SwDeviceBufs& b, cudaStream_t st,
-                      cudaEvent_t ev0, cudaEvent_t ev1, float* class_ms, std::string& err);
+                      const SwFork* fork, cudaEvent_t ev0, cudaEvent_t ev1, float* class_ms, std::string& err);
 
 struct SwArenaLayout;
 
@@ -218,6 +274,9 @@ private:
     int dev_ = 0;
     cudaStream_t stream_ = nullptr;
     cudaEvent_t ev_[2] = {};
+    cudaStream_t side_[kSwGroups] = {};
+    cudaEvent_t ev_side_[kSwGroups] = {}, ev_fork_ = nullptr;
+    SwFork fork_;
     void* arena_ = nullptr;
     size_t arena_bytes_ = 0;
     void* pinned_ = nullptr;
