@@ -636,7 +636,7 @@ constexpr uint64_t kSwScratchCap = 6ull << 30;
 // at a fraction of the memory bandwidth, and the bases of a genome-scale batch are ~100 MB).
 void staged_copy(void* dst, const void* src, size_t bytes)
 {
-    constexpr size_t kPerThread = 8u << 20;
+    constexpr size_t kPerThread = 2u << 20;
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const unsigned nt = (unsigned)std::min<size_t>({hw, 8u, bytes / kPerThread});
     if (nt <= 1) {
@@ -714,20 +714,33 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
     p = SwPlan();
     p.n = n;
     p.cigar_cap = std::min<uint32_t>(cigar_cap, kSwMaxSeq - 1);
-    std::vector<uint8_t> grp(n);
+    // 16-bit group of every multiple of 32 columns, where the parameters allow one (the rule depends on
+    // an alignment only through its class and the length limit); -1: sw_class_of decides
+    constexpr uint32_t kMaxK16 = 24;
+    int8_t group16[kMaxK16 + 1];
+    for (uint32_t k = 0; k <= kMaxK16; ++k) {
+        const int c = sw_class_of(prm, 1, 1, 32 * k);
+        group16[k] = (int8_t)(sw_packs(prm, 1, 32 * k, kSwK[c]) ? c : -1);
+    }
+    constexpr uint32_t kBuckets = 1024;
+    std::vector<uint32_t> key(n);
     uint32_t counts[kSwGroups] = {};
     p.slot_off.resize(n);
     for (uint32_t q = 0; q < n; ++q) {
-        const int c = sw_class_of(prm, variant, nrow[q], ncol[q]);
-        const bool packs = c != kSwWrapClass && sw_packs(prm, nrow[q], ncol[q], kSwK[c]);
-        const int g = packs ? c : kSwWrapClass + c;
-        grp[q] = (uint8_t)g;
+        const uint32_t R = nrow[q], C = ncol[q], k = (C + 31) / 32;
+        const bool fits = std::max(R, C) < (uint32_t)kSwMaxSeq;
+        const int g16 = k <= kMaxK16 && R < (uint32_t)kSwMaxSeq ? group16[k] : -1;
+        const int g = g16 >= 0 ? g16 : kSwWrapClass + sw_class_of(prm, variant, R, C);
         ++counts[g];
-        p.max_rows[g] = std::max(p.max_rows[g], nrow[q]);
-        p.cells += (uint64_t)nrow[q] * ncol[q];
+        p.max_rows[g] = std::max(p.max_rows[g], R);
+        p.cells += (uint64_t)R * C;
         p.slot_off[q] = p.slots;
-        if (std::max(nrow[q], ncol[q]) < (uint32_t)kSwMaxSeq)  // runs <= rows + columns consumed
-            p.slots += std::min<uint64_t>(p.cigar_cap, (uint64_t)nrow[q] + ncol[q]);
+        if (fits) p.slots += std::min<uint64_t>(p.cigar_cap, (uint64_t)R + C);  // runs <= rows + columns consumed
+        // by group, then longest first in buckets: two rows in the 16-bit groups, whose warps run
+        // neighbours together for the longer one's rows, 4096 cells in the others (there the order only
+        // balances the persistent warps' load)
+        const uint64_t len = g16 >= 0 ? R >> 1 : ((uint64_t)R * C) >> 12;
+        key[q] = (uint32_t)g * kBuckets + (kBuckets - 1 - (uint32_t)std::min<uint64_t>(kBuckets - 1, len));
     }
     if (p.slots > 0xffffffffull) {
         err = "Smith-Waterman batch needs more than 2^32 CIGAR ops of room: split it";
@@ -735,19 +748,11 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
     }
     p.begin[0] = 0;
     for (int g = 0; g < kSwGroups; ++g) p.begin[g + 1] = p.begin[g] + counts[g];
-    // one counting sort: by group, then longest first in buckets: two rows in the 16-bit groups, whose
-    // warps run neighbours together for the longer one's rows, 4096 cells in the others (there the
-    // order only balances the persistent warps' load)
-    constexpr uint32_t kBuckets = 1024;
-    auto key = [&](uint32_t q) {
-        const uint64_t len = grp[q] < kSwWrapClass ? nrow[q] >> 1 : ((uint64_t)nrow[q] * ncol[q]) >> 12;
-        return (uint32_t)grp[q] * kBuckets + (kBuckets - 1 - (uint32_t)std::min<uint64_t>(kBuckets - 1, len));
-    };
     std::vector<uint32_t> start((size_t)kSwGroups * kBuckets + 1, 0);
-    for (uint32_t q = 0; q < n; ++q) ++start[key(q) + 1];
+    for (uint32_t q = 0; q < n; ++q) ++start[key[q] + 1];
     for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
     p.order.assign(n, 0);
-    for (uint32_t q = 0; q < n; ++q) p.order[start[key(q)]++] = q;
+    for (uint32_t q = 0; q < n; ++q) p.order[start[key[q]]++] = q;
     uint64_t need[kSwGroups] = {}, sum = 0, most = 0;
     for (int g = 0; g < kSwGroups; ++g) {
         const uint32_t m = counts[g];
@@ -986,8 +991,30 @@ phmm_status SwAligner::align(const SwParams& prm, int variant, uint32_t n, const
     if (st != PHMM_OK) return st;
     std::lock_guard<std::mutex> lk(mu_);
     SW_CK(cudaSetDevice(dev_));
+    // inputs through pinned staging in one copy: items | order | slot offsets | haplotypes | reads, the
+    // bases staged while the batch is planned (the inputs' layout does not depend on the plan)
+    const SwArenaLayout in(n, hap_bytes, read_bytes, 0, 0);
+    st = ensure_pinned(in.in_bytes(), err);
+    if (st != PHMM_OK) return st;
+    uint8_t* h = (uint8_t*)pinned_;
+    auto stage = [&] {
+        staged_copy(h + in.items, items, sizeof(SwItem) * (size_t)n);
+        if (hap_bytes) staged_copy(h + in.hap, hap, hap_bytes);
+        if (read_bytes) staged_copy(h + in.read, read, read_bytes);
+    };
     SwPlan p;
-    st = plan(prm, variant, n, items, cigar_cap, p, err);
+    {
+        std::thread helper;
+        if (hap_bytes + read_bytes >= (1u << 20)) helper = std::thread(stage);
+        else stage();
+        try {
+            st = plan(prm, variant, n, items, cigar_cap, p, err);
+        } catch (...) {
+            if (helper.joinable()) helper.join();
+            throw;
+        }
+        if (helper.joinable()) helper.join();
+    }
     if (st != PHMM_OK) return st;
     const SwArenaLayout L(n, hap_bytes, read_bytes, p.slots, p.scratch);
     if (L.bytes > arena_bytes_) {
@@ -1005,16 +1032,9 @@ phmm_status SwAligner::align(const SwParams& prm, int variant, uint32_t n, const
         }
         arena_bytes_ = sz;
     }
-    // inputs through pinned staging in one copy: items | order | slot offsets | haplotypes | reads
-    st = ensure_pinned(L.in_bytes(), err);
-    if (st != PHMM_OK) return st;
-    uint8_t* h = (uint8_t*)pinned_;
     uint8_t* d = (uint8_t*)arena_;
-    staged_copy(h + L.items, items, sizeof(SwItem) * (size_t)n);
     std::memcpy(h + L.order, p.order.data(), 4ull * n);
     std::memcpy(h + L.slot_off, p.slot_off.data(), 8ull * n);
-    if (hap_bytes) staged_copy(h + L.hap, hap, hap_bytes);
-    if (read_bytes) staged_copy(h + L.read, read, read_bytes);
     SW_CK(cudaMemcpyAsync(d, h, L.in_bytes(), cudaMemcpyHostToDevice, stream_));
     SW_CK(cudaEventRecord(ev_[0], stream_));
     st = sw_launch(p, prm, variant, L.bufs(d), stream_, &fork_, nullptr, nullptr, nullptr, err);

@@ -36,8 +36,32 @@ def _u8(x) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(x, dtype=np.uint8))
 
 
+def _addr(a: np.ndarray) -> int:
+    return a.__array_interface__["data"][0]
+
+
 def _ptr(a: np.ndarray | None):
-    return None if a is None else a.ctypes.data_as(C.c_void_p)
+    return None if a is None else C.c_void_p(_addr(a))
+
+
+def _join(parts: Iterable) -> tuple[np.ndarray, np.ndarray, np.ndarray]:
+    """Sequences end to end in one (writable) array, their offsets and their lengths.  Byte strings, what
+    a caller usually holds, are joined in one call; other kinds are converted one by one."""
+    parts = list(parts)
+    if {bytes, bytearray}.issuperset(map(type, parts)):
+        flat = np.frombuffer(bytearray().join(parts), np.uint8) if any(parts) else np.zeros(0, np.uint8)
+    else:
+        parts = [_u8(p) for p in parts]
+        flat = np.concatenate(parts)
+    lens = np.fromiter(map(len, parts), np.uint64, len(parts))
+    off = np.zeros(lens.size + 1, np.uint64)
+    lens.cumsum(out=off[1:])
+    return flat, off, lens
+
+
+def _mapq(mapq, n: int) -> np.ndarray:
+    mq = np.ascontiguousarray(np.asarray(mapq, np.uint8).reshape(-1))
+    return np.full(n, mq[0], np.uint8) if mq.size == 1 and n > 1 else mq
 
 
 @dataclass
@@ -114,19 +138,16 @@ class PackedBatch:
     @classmethod
     def from_regions(cls, regions: Iterable[Region]) -> "PackedBatch":
         regions = list(regions)
-        haps = [_u8(h) for r in regions for h in r.haplotypes]
-        reads = [_u8(x) for r in regions for x in r.reads]
-        cat = lambda parts: np.concatenate(parts) if parts else np.zeros(0, np.uint8)
-        qual = [_u8(x) for r in regions for x in r.quality]
-        ins = [_u8(x) for r in regions for x in r.insertion_qualities]
-        dele = [_u8(x) for r in regions for x in r.deletion_qualities]
-        gcp = [_u8(x) for r in regions for x in r.gap_contiguous_qualities]
-        for arr in (qual, ins, dele, gcp):
-            if [len(a) for a in arr] != [len(a) for a in reads]:
+        haps, hap_off, _ = _join([h for r in regions for h in r.haplotypes])
+        reads, read_off, lens = _join([x for r in regions for x in r.reads])
+        arrays = []
+        for name in ("quality", "insertion_qualities", "deletion_qualities", "gap_contiguous_qualities"):
+            arr, _, n = _join([x for r in regions for x in getattr(r, name)])
+            if not np.array_equal(n, lens):
                 raise ValueError("every quality array must have its read's length")
-        off = lambda parts: np.concatenate([[0], np.cumsum([len(p) for p in parts])]).astype(np.uint64)
+            arrays.append(arr)
         return cls(np.array([r.n_haps for r in regions], np.uint32), np.array([r.n_reads for r in regions], np.uint32),
-                   cat(haps), off(haps), cat(reads), cat(qual), cat(ins), cat(dele), cat(gcp), off(reads))
+                   haps, hap_off, reads, *arrays, read_off)
 
     def pinned(self) -> "PackedBatch":
         """A copy whose arrays live in page-locked host memory (fast DMA); uses torch for the pinning."""
@@ -357,22 +378,18 @@ class Engine:
                     pcr_option: str | int = "CONSERVATIVE"):
         """call_pairhmm semantics; returns (matrix [n_haps][n_reads] with kept reads first, keep mask)."""
         pcr = PCR_MODELS[pcr_option] if isinstance(pcr_option, str) else int(pcr_option)
-        hs = [_u8(h) for h in haplotypes]
-        rs = [_u8(r) for r in reads]
-        qs = [_u8(q) for q in base_quals]
-        cat = lambda parts: np.concatenate(parts) if parts else np.zeros(1, np.uint8)
-        off = lambda parts: np.concatenate([[0], np.cumsum([len(p) for p in parts])]).astype(np.uint64)
-        hb, hoff, rb, roff, qb = cat(hs), off(hs), cat(rs), off(rs), cat(qs)
-        mq = np.ascontiguousarray(np.asarray(mapq, np.uint8).reshape(-1))
-        if mq.size == 1 and len(rs) > 1:
-            mq = np.full(len(rs), mq[0], np.uint8)
-        out = np.empty(len(hs) * len(rs), np.float64)
-        keep = np.empty(len(rs), np.uint8)
+        hb, hoff, hl = _join(haplotypes)
+        rb, roff, rl = _join(reads)
+        qb, _, _ = _join(base_quals)
+        n_haps, n_reads = hl.size, rl.size
+        mq = _mapq(mapq, n_reads)
+        out = np.empty(n_haps * n_reads, np.float64)
+        keep = np.empty(n_reads, np.uint8)
         nk = C.c_uint32()
-        st = self._lib.phmm_call_region(self._h, len(hs), _ptr(hb), _ptr(hoff), len(rs), _ptr(rb), _ptr(qb), _ptr(roff),
+        st = self._lib.phmm_call_region(self._h, n_haps, _ptr(hb), _ptr(hoff), n_reads, _ptr(rb), _ptr(qb), _ptr(roff),
                                         _ptr(mq), int(min_quality_threshold), pcr, _ptr(out), _ptr(keep), C.byref(nk))
         check(st)
-        return out.reshape(len(hs), len(rs)), keep.astype(bool)
+        return out.reshape(n_haps, n_reads), keep.astype(bool)
 
 
 class RegionTicket:
@@ -381,23 +398,17 @@ class RegionTicket:
     def __init__(self, engine: Engine, haplotypes, reads, base_quals, mapq, min_quality_threshold, pcr_option,
                  events=None, want_matrix: bool = True, want_allele_lk: bool = False, realign=None):
         pcr = PCR_MODELS[pcr_option] if isinstance(pcr_option, str) else int(pcr_option)
-        hs = [_u8(h) for h in haplotypes]
-        rs = [_u8(r) for r in reads]
-        qs = [_u8(q) for q in base_quals]
-        cat = lambda parts: np.concatenate(parts) if parts else np.zeros(1, np.uint8)
-        off = lambda parts: np.concatenate([[0], np.cumsum([len(p) for p in parts])]).astype(np.uint64)
-        self._keepalive = [cat(hs), off(hs), cat(rs), off(rs), cat(qs)]
-        hb, hoff, rb, roff, qb = self._keepalive
-        mq = np.ascontiguousarray(np.asarray(mapq, np.uint8).reshape(-1))
-        if mq.size == 1 and len(rs) > 1:
-            mq = np.full(len(rs), mq[0], np.uint8)
-        self._keepalive.append(mq)
-        self.n_haps, self.n_reads = len(hs), len(rs)
+        hb, hoff, hap_lens = _join(haplotypes)
+        rb, roff, read_lens = _join(reads)
+        qb, _, _ = _join(base_quals)
+        self.n_haps, self.n_reads = hap_lens.size, read_lens.size
+        mq = _mapq(mapq, self.n_reads)
+        self._keepalive = [hb, hoff, rb, roff, qb, mq]
         self.out = np.empty(self.n_haps * self.n_reads, np.float64) if want_matrix else None
         self.keep = np.empty(max(self.n_reads, 1), np.uint8)
         self.n_kept = C.c_uint32()
-        inp = _lib.RegionInput(self.n_haps, hb.ctypes.data, hoff.ctypes.data, self.n_reads, rb.ctypes.data,
-                               qb.ctypes.data, roff.ctypes.data, mq.ctypes.data, int(min_quality_threshold), pcr)
+        inp = _lib.RegionInput(self.n_haps, _addr(hb), _addr(hoff), self.n_reads, _addr(rb),
+                               _addr(qb), _addr(roff), _addr(mq), int(min_quality_threshold), pcr)
         self.events = None
         ev_ptr = None
         if events:
@@ -408,9 +419,9 @@ class RegionTicket:
             self.best = np.empty(len(na), np.int32)
             self.allele_lk = np.empty(max(int(na.astype(np.int64).sum()) * self.n_reads, 1)) if want_allele_lk else None
             self._keepalive += [na, ha]
-            self.events = _lib.RegionEvents(len(na), na.ctypes.data, ha.ctypes.data, self.gl.ctypes.data,
-                                            self.best.ctypes.data,
-                                            self.allele_lk.ctypes.data if want_allele_lk else None)
+            self.events = _lib.RegionEvents(len(na), _addr(na), _addr(ha), _addr(self.gl),
+                                            _addr(self.best),
+                                            _addr(self.allele_lk) if want_allele_lk else None)
             self._n_alleles = na
             ev_ptr = C.byref(self.events)
         self._engine = engine
@@ -425,17 +436,17 @@ class RegionTicket:
             cr = np.ascontiguousarray(np.asarray(realign.get("clip_right", zeros), np.uint16).reshape(-1))
             if prio.size != self.n_haps or cl.size != self.n_reads or cr.size != self.n_reads:
                 raise ValueError("realign: one priority per haplotype and one clip per read")
-            lens = np.array([len(r) for r in rs], np.int64)
-            cap = int(np.minimum(lens - cl - cr + max((len(h) for h in hs), default=0), sw.MAX_CIGAR).sum())
+            longest = int(hap_lens.max()) if self.n_haps else 0
+            cap = int(np.minimum(read_lens.astype(np.int64) - cl - cr + longest, sw.MAX_CIGAR).sum())
             cap = int(realign.get("cigar_capacity", cap))
             self.best_hap = np.empty(max(self.n_reads, 1), np.int32)
             self.sw_res = np.zeros(max(self.n_reads, 1), sw.SW_RESULT_DTYPE)
             self.cigars = np.empty(max(cap, 1), np.uint32)
             self.cigar_total = C.c_uint64()
             self._keepalive += [prio, cl, cr]
-            self.realign = _lib.RegionRealign(prio.ctypes.data, cl.ctypes.data, cr.ctypes.data,
-                                              self.best_hap.ctypes.data, self.sw_res.ctypes.data,
-                                              self.cigars.ctypes.data, self.cigars.size,
+            self.realign = _lib.RegionRealign(_addr(prio), _addr(cl), _addr(cr),
+                                              _addr(self.best_hap), self.sw_res.ctypes.data,
+                                              _addr(self.cigars), self.cigars.size,
                                               C.cast(C.byref(self.cigar_total), C.c_void_p))
             check(engine._lib.phmm_submit_region_realign(engine._h, C.byref(inp), ev_ptr, C.byref(self.realign),
                                                          _ptr(self.out), _ptr(self.keep), C.byref(self.n_kept),
