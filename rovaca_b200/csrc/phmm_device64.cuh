@@ -13,6 +13,8 @@
 // instead of 4 K + 3, two shuffles instead of three, and (PM_EQ) 7 operations per cell instead of 8.
 #pragma once
 
+#include <type_traits>
+
 #include "phmm_device.cuh"
 
 namespace phmm {
@@ -220,14 +222,13 @@ __device__ __forceinline__ double row_diag(const LaneRowsRow<K>& L, int k, doubl
     return diag_eq<V, true>(L.gm[k], L.mm[k], dgM, dgI, dgD);
 }
 
-// Whether every nonzero input of the lane's next PHMM_F64_VOTE_EVERY steps reaches
-// flush_free_hi<K>(): its rows' pending sums and next-column D, and the two values it hands the lane
+// Whether every nonzero input of the lane's next STEPS steps reaches flush_free_hi<K, STEPS>(): its rows' pending sums and next-column D, and the two values it hands the lane
 // below (that lane's first-row inputs).  The longest product chain of a step is still K + 1 factors
 // (the insertion chain from the first row's M down to the value handed on), so the bound of
 // rows_flush_free holds.
 // The minimum is taken as a tree (depth log2(2 K + 2) instead of a chain of 2 K + 2 dependent
 // operations): the next step's arithmetic waits on this vote.
-template <int K, typename LR>
+template <int K, int STEPS, typename LR>
 __device__ __forceinline__ bool rows_flush_free_eq(const LR& L)
 {
     constexpr int N = 2 * K + 2;
@@ -244,7 +245,7 @@ __device__ __forceinline__ bool rows_flush_free_eq(const LR& L)
 #pragma unroll
         for (int i = 0; i + w < N; i += 2 * w) v[i] = min(v[i], v[i + w]);
     }
-    return v[0] >= flush_free_hi<K>() - 1u;
+    return v[0] >= flush_free_hi<K, STEPS>() - 1u;
 }
 
 // Sweep one stripe over the column stream of haplotypes [g_lo, g_hi): as `sweep` (phmm_device.cuh),
@@ -265,7 +266,12 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
     double D0 = 0.0;
     double Stop = 0.0;  // lane 0's first-row sum below the boundary row (M = I = 0, D = C/H)
     double sumM = 0.0, sumI = 0.0;
-    bool flush_free = false;  // the current step's inputs are all 0 or above the bound
+    // flush_free: the current two steps' inputs are all 0 or above the bound.  The vote for the next two
+    // is taken after the first of these, on the bound of three steps, so that the second step's
+    // arithmetic covers its latency (the branch below waits on it): 26.5 against 27.6 ms for the FP64
+    // pass of 60 underflow-stress regions with a vote after every second step and a branch per step.
+    bool flush_free = false, free_next = false;
+    uint32_t wn = codes[-lane];  // the code word of the lane's next column, loaded a step ahead (26.1 ms)
 
     const int steps = Tcols + kWarp;
 
@@ -304,7 +310,9 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
         }
     };
 
-    auto step = [&](int t, bool check) {
+    constexpr bool kVote = PHMM_F64_VOTE && !FROM_SCR;
+    auto step = [&](int t, bool check, auto flush) {
+        constexpr bool FL = decltype(flush)::value;
         const int p = t - lane;
         double uI = shfl_up1(L.In);
         double uS = shfl_up1(L.Sn);
@@ -320,7 +328,8 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
                 uS = Stop;
             }
         }
-        const uint32_t w = codes[p];
+        const uint32_t w = wn;
+        wn = codes[p + 1];
         const uint32_t cls = (w & kTabMask) >> kTabShift;
         double pr[K];
 #pragma unroll
@@ -333,11 +342,7 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
                 if (i >= 0 && i < R && b.read_bases[roff + i] == hb) pr[k] = tb.pmat[b.read_q[roff + i] & 127];
             }
         }
-        constexpr bool kVote = PHMM_F64_VOTE && !FROM_SCR;
-        if (kVote && flush_free)
-            cells_eq<K, V, false>(L, pr, uI, uS);
-        else
-            cells_eq<K, V, true>(L, pr, uI, uS);
+        cells_eq<K, V, FL>(L, pr, uI, uS);
         if (TO_SCR) {
             if (lane == kWarp - 1 && p >= 0 && p < Tcols) {
                 scr[2 * p + 0] = L.In;
@@ -347,19 +352,34 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
             sumM = radd(sumM, L.Mb);
             sumI = radd(sumI, L.Ib);
         }
-        if constexpr (kVote)
-            if (PHMM_F64_VOTE_EVERY == 1 || t % PHMM_F64_VOTE_EVERY == PHMM_F64_VOTE_EVERY - 1)
-                flush_free = __all_sync(0xffffffffu, rows_flush_free_eq<K>(L));
+        if constexpr (kVote) {
+            if (t % 2 == 0) free_next = __all_sync(0xffffffffu, rows_flush_free_eq<K, 3>(L));
+            else flush_free = free_next;
+        }
     };
+    static_assert(kChunkScalar % 2 == 0, "steps run in pairs");
+    const auto yes = std::true_type{};
+    const auto no = std::false_type{};
 
     for (int t0 = 0; t0 < steps; t0 += kChunkScalar) {
         const int nb31 = __shfl_sync(0xffffffffu, nb, kWarp - 1);
         if (nb31 >= t0 + kChunkScalar && t0 + kChunkScalar <= steps) {
 #pragma unroll
-            for (int u = 0; u < kChunkScalar; ++u) step(t0 + u, false);
+            for (int u = 0; u < kChunkScalar; u += 2) {
+                if (kVote && flush_free) {
+                    step(t0 + u, false, no);
+                    step(t0 + u + 1, false, no);
+                } else {
+                    step(t0 + u, false, yes);
+                    step(t0 + u + 1, false, yes);
+                }
+            }
         } else {
             for (int u = 0; u < kChunkScalar; ++u)
-                if (t0 + u < steps) step(t0 + u, true);
+                if (t0 + u < steps) {
+                    if (kVote && flush_free) step(t0 + u, true, no);
+                    else step(t0 + u, true, yes);
+                }
         }
     }
 }
