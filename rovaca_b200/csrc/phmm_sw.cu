@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(32 * kSwBlockWarps, sw_min_blocks<K>()) sw_ker
 
 // Two alignments per warp (phmm_sw16.cuh): one-warp blocks, each claiming pairs of neighbours in the
 // launch's order (longest haplotype first, so that the two are of about one length).
-template <int K>
+template <int K, bool REB>
 __global__ void __launch_bounds__(32, K <= 12 ? 16 : 12) sw16_kernel(SwView v, uint32_t max_rows)
 {
     extern __shared__ uint4 sw16_shared[];
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(32, K <= 12 ? 16 : 12) sw16_kernel(SwView v, u
         if (lane == 0) p = atomicAdd(v.claim, 1u);
         p = __shfl_sync(kFull, p, 0);
         if (2 * p >= v.n) break;
-        sw16_pair<K>(v, v.order[2 * p], 2 * p + 1 < v.n ? v.order[2 * p + 1] : 0xffffffffu, lane, scr, (char*)sw16_shared,
+        sw16_pair<K, REB>(v, v.order[2 * p], 2 * p + 1 < v.n ? v.order[2 * p + 1] : 0xffffffffu, lane, scr, (char*)sw16_shared,
                      max_rows);
     }
 }
@@ -521,28 +521,19 @@ __global__ void __launch_bounds__(kRealignThreads) realign_items_kernel(RealignV
 }
 
 using Sw16Kernel = void (*)(SwView, uint32_t);
-const Sw16Kernel kSw16Kernels[kSwWrapClass] = {
-    sw16_kernel<1>, sw16_kernel<2>, sw16_kernel<3>,  sw16_kernel<4>,  sw16_kernel<5>,  sw16_kernel<6>,  sw16_kernel<7>,
-    sw16_kernel<8>, sw16_kernel<10>, sw16_kernel<12>, sw16_kernel<16>, sw16_kernel<20>, sw16_kernel<24>,
-};
-uint32_t sw16_shared_bytes(int c, uint32_t max_rows)
+#define PHMM_SW16_WIDTHS(F, REB)                                                                                   \
+    F<1, REB>, F<2, REB>, F<3, REB>, F<4, REB>, F<5, REB>, F<6, REB>, F<7, REB>, F<8, REB>, F<10, REB>, F<12, REB>, \
+        F<16, REB>, F<20, REB>, F<24, REB>
+const Sw16Kernel kSw16Kernels[kSwPairGroups] = {PHMM_SW16_WIDTHS(sw16_kernel, false),
+                                                PHMM_SW16_WIDTHS(sw16_kernel, true)};
+template <int K, bool REB>
+uint32_t sw16_bytes(uint32_t max_rows)
 {
-    switch (kSwK[c]) {
-    case 1: return Sw16Shared<1>::bytes(max_rows);
-    case 2: return Sw16Shared<2>::bytes(max_rows);
-    case 3: return Sw16Shared<3>::bytes(max_rows);
-    case 4: return Sw16Shared<4>::bytes(max_rows);
-    case 5: return Sw16Shared<5>::bytes(max_rows);
-    case 6: return Sw16Shared<6>::bytes(max_rows);
-    case 7: return Sw16Shared<7>::bytes(max_rows);
-    case 8: return Sw16Shared<8>::bytes(max_rows);
-    case 10: return Sw16Shared<10>::bytes(max_rows);
-    case 12: return Sw16Shared<12>::bytes(max_rows);
-    case 16: return Sw16Shared<16>::bytes(max_rows);
-    case 20: return Sw16Shared<20>::bytes(max_rows);
-    default: return Sw16Shared<24>::bytes(max_rows);
-    }
+    return Sw16Shared<K, REB>::bytes(max_rows);
 }
+using Sw16Bytes = uint32_t (*)(uint32_t);
+const Sw16Bytes kSw16Bytes[kSwPairGroups] = {PHMM_SW16_WIDTHS(sw16_bytes, false), PHMM_SW16_WIDTHS(sw16_bytes, true)};
+#undef PHMM_SW16_WIDTHS
 
 using SwKernel = void (*)(SwView);
 
@@ -693,9 +684,9 @@ phmm_status device_info(int device, SwDeviceInfo& out, std::string& err)
             SW_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kSwKernels[c], 32 * kSwBlockWarps, 0));
             di.occ[c] = std::max(b, 1);
         }
-        for (int c = 0; c < kSwWrapClass; ++c)
-            SW_CK(cudaFuncSetAttribute(kSw16Kernels[c], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sw16_shared_bytes(c, kSwMaxSeq - 1)));
+        for (int g = 0; g < kSwPairGroups; ++g)
+            SW_CK(cudaFuncSetAttribute(kSw16Kernels[g], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kSw16Bytes[g](kSwMaxSeq - 1)));
         SW_CK(cudaSetDevice(cur));
         di.ready = true;
     }
@@ -714,13 +705,17 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
     p = SwPlan();
     p.n = n;
     p.cigar_cap = std::min<uint32_t>(cigar_cap, kSwMaxSeq - 1);
-    // 16-bit group of every multiple of 32 columns, where the parameters allow one (the rule depends on
-    // an alignment only through its class and the length limit); -1: sw_class_of decides
+    // two-per-warp group of every multiple of 32 columns, where the parameters allow one, for alignments
+    // of the reference's int16 and int32 kernels (sw_form depends on an alignment only through its class,
+    // its kernel and the length limit); -1: sw_class_of decides
     constexpr uint32_t kMaxK16 = 24;
-    int8_t group16[kMaxK16 + 1];
+    int8_t group16[2][kMaxK16 + 1];
     for (uint32_t k = 0; k <= kMaxK16; ++k) {
         const int c = sw_class_of(prm, 1, 1, 32 * k);
-        group16[k] = (int8_t)(sw_packs(prm, 1, 32 * k, kSwK[c]) ? c : -1);
+        for (int i32 = 0; i32 < 2; ++i32) {
+            const SwForm f = sw_form(prm, i32 != 0, 1, 32 * k, kSwK[c]);
+            group16[i32][k] = (int8_t)(f == kSwOnePerWarp ? -1 : f * kSwWrapClass + c);
+        }
     }
     constexpr uint32_t kBuckets = 1024;
     std::vector<uint32_t> key(n);
@@ -729,8 +724,16 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
     for (uint32_t q = 0; q < n; ++q) {
         const uint32_t R = nrow[q], C = ncol[q], k = (C + 31) / 32;
         const bool fits = std::max(R, C) < (uint32_t)kSwMaxSeq;
-        const int g16 = k <= kMaxK16 && R < (uint32_t)kSwMaxSeq ? group16[k] : -1;
-        const int g = g16 >= 0 ? g16 : kSwWrapClass + sw_class_of(prm, variant, R, C);
+        int g16 = -1;
+        if (k <= kMaxK16 && R < (uint32_t)kSwMaxSeq) g16 = group16[sw_uses_int32(variant, R, C, prm.match)][k];
+        int g = g16;
+        if (g16 < 0 || g16 >= kSwWrapClass) {  // (a plain 16-bit score cannot wrap the int16 kernel)
+            const int c = sw_class_of(prm, variant, R, C);
+            if (g16 < 0 || c == kSwWrapClass) {
+                g = kSwPairGroups + c;
+                g16 = -1;
+            }
+        }
         ++counts[g];
         p.max_rows[g] = std::max(p.max_rows[g], R);
         p.cells += (uint64_t)R * C;
@@ -759,10 +762,9 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
         if (m == 0) continue;
         const int c = sw_group_class(g);
         uint64_t blocks, warps;
-        if (g < kSwWrapClass) {
+        if (g < kSwPairGroups) {
             int occ = 0;
-            SW_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kSw16Kernels[c], 32,
-                                                                sw16_shared_bytes(c, p.max_rows[g])));
+            SW_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kSw16Kernels[g], 32, kSw16Bytes[g](p.max_rows[g])));
             p.stride[g] = std::max<uint64_t>(256, sw16_layout(p.max_rows[g], kSwK[c]).total);
             blocks = std::min<uint64_t>(((uint64_t)m + 1) / 2, (uint64_t)std::max(occ, 1) * di.sms);
             warps = 1;
@@ -827,8 +829,8 @@ phmm_status sw_launch(const SwPlan& p, const SwParams& prm, int variant, const S
         const cudaStream_t s = side ? fork->side[g] : st;
         if (side) SW_CK(cudaStreamWaitEvent(s, fork->fork, 0));
         if (class_ms) SW_CK(cudaEventRecord(ev0, s));
-        if (g < kSwWrapClass)
-            kSw16Kernels[c]<<<p.grid[g], 32, sw16_shared_bytes(c, p.max_rows[g]), s>>>(v, p.max_rows[g]);
+        if (g < kSwPairGroups)
+            kSw16Kernels[g]<<<p.grid[g], 32, kSw16Bytes[g](p.max_rows[g]), s>>>(v, p.max_rows[g]);
         else
             kSwKernels[c]<<<p.grid[g], 32 * kSwBlockWarps, 0, s>>>(v);
         SW_CK(cudaGetLastError());

@@ -33,9 +33,10 @@ constexpr int kSwClasses = 14;       // 13 stripe widths (kSwK) + the 16-bit wra
 constexpr int kSwWrapClass = 13;
 constexpr int kSwK[kSwClasses] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16, 20, 24, 24};
 // Kernel launches of a batch: the 13 stripe widths with two alignments per warp in 16-bit halves
-// (phmm_sw16.cuh), then the 14 classes with one alignment per warp.
-constexpr int kSwGroups = kSwWrapClass + kSwClasses;
-PHMM_HD inline int sw_group_class(int g) { return g < kSwWrapClass ? g : g - kSwWrapClass; }
+// (phmm_sw16.cuh), the same in its rebased form, then the 14 classes with one alignment per warp.
+constexpr int kSwPairGroups = 2 * kSwWrapClass;
+constexpr int kSwGroups = kSwPairGroups + kSwClasses;
+PHMM_HD inline int sw_group_class(int g) { return g < kSwPairGroups ? g % kSwWrapClass : g - kSwPairGroups; }
 
 // What one class launch works on.
 struct SwView {
@@ -119,18 +120,26 @@ PHMM_HD inline int sw16_bias(const SwParams& p, int K)
 {
     return -(2 * p.gap_open + p.mismatch + (32 * K + 2) * p.gap_extend) + 16;
 }
-// Whether alignments of at most 32 * K read bases run two per warp in 16-bit halves: parameters for
-// which pad columns stand for the boundary (gap_open <= 0, gap_extend < 0, mismatch <= 0 <= match), a
-// bias under 8,000 (E then stays above the reference's 16-bit cutoff of -8192, which can change
-// nothing, see sw_cutoff_can_bind) and scores that fit 15 bits with it.
-inline bool sw_packs(const SwParams& p, uint32_t nrow, uint32_t ncol, int K)
+// How alignments of at most 32 * K read bases run: 16-bit halves, rebased 16-bit halves, or one per warp.
+// Both two-per-warp forms need parameters for which pad columns stand for the boundary (gap_open <= 0,
+// gap_extend < 0, mismatch <= 0 <= match) and, where the reference takes its int16 kernel, a bias under
+// 8,000 (E then stays above that kernel's cutoff of -8192, which can change nothing, see
+// sw_cutoff_can_bind; its adds cannot wrap either, or the alignment is in the wrap-around class).  The
+// plain form needs scores that fit 15 bits with the bias; the rebased form needs what a lane holds to stay
+// within 15 bits of its base from one rebasing to the next (kSw16Rebase = 32 rows).
+enum SwForm { kSwPlain16 = 0, kSwRebased16 = 1, kSwOnePerWarp = 2 };
+inline SwForm sw_form(const SwParams& p, bool i32, uint32_t nrow, uint32_t ncol, int K)
 {
-    if (ncol > 32u * (uint32_t)K || nrow >= (uint32_t)kSwMaxSeq) return false;
+    if (ncol > 32u * (uint32_t)K || nrow >= (uint32_t)kSwMaxSeq) return kSwOnePerWarp;
     if (p.gap_open > 0 || p.gap_open < -4000 || p.gap_extend >= 0 || p.gap_extend < -4000 || p.mismatch > 0 ||
         p.mismatch < -8000 || p.match < 0 || p.match > 32000)
-        return false;
+        return kSwOnePerWarp;
     const int bias = sw16_bias(p, K);
-    return bias < 8000 && bias + (32 * K + 1) * (long long)p.match <= 32000;
+    if (bias < 8000 && bias + (32 * K + 1) * (long long)p.match <= 32000) return kSwPlain16;
+    if (!i32 && bias >= 8000) return kSwOnePerWarp;
+    const long long reach = (K + 1 + 32) * (long long)(p.match - p.gap_open) +
+                            2ll * (p.match - p.mismatch - p.gap_open - p.gap_extend);
+    return reach <= 32000 ? kSwRebased16 : kSwOnePerWarp;
 }
 
 int sw_class_of(const SwParams& prm, int variant, uint32_t nrow, uint32_t ncol);
@@ -146,7 +155,7 @@ struct SwPlan {
     uint32_t begin[kSwGroups + 1] = {};
     uint64_t stride[kSwGroups] = {};         // scratch bytes per warp of each group
     uint64_t scratch_off[kSwGroups] = {};    // its scratch
-    uint32_t max_rows[kSwGroups] = {};       // longest haplotype of the group (16-bit groups)
+    uint32_t max_rows[kSwGroups] = {};       // longest haplotype of the group (two-per-warp groups)
     int grid[kSwGroups] = {};
     bool concurrent = true;                  // the groups have disjoint scratch and may run together
     int gather_blocks = 1;

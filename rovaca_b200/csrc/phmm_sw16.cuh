@@ -1,8 +1,9 @@
 // Smith-Waterman of two alignments per warp in 16-bit halves.  The recurrences, tie rules, end-cell
 // choice and trace-back are those of phmm_sw.cu (reference: common/base/lib/ro_sw/sw_core_template.h:
-// 111-352, sw_cigar.c:22-171); this is the form for alignments whose scores fit 16 bits whatever the
-// bases (sw_packs below: the genotyping parameters up to 768 read bases), so that the reference's
-// int16 and int32 kernels give the same results and no add can wrap.
+// 111-352, sw_cigar.c:22-171); this is the form for alignments whose scores, or whose scores' differences
+// within a lane, fit 16 bits whatever the bases (sw_form: the genotyping and the assembly parameters up to
+// 768 read bases), so that no add can wrap and the reference's int16 and int32 kernels give the same
+// results.
 //
 // Mapping.  Alignment X in the low and Y in the high half of every 32-bit register.  Lane l holds K
 // read columns of both and works on row t + 1 - l at step t; the left neighbour's H and E arrive by one
@@ -89,17 +90,22 @@ PHMM_HD inline uint32_t sw16_class(uint8_t b)
     return b == 'A' ? 0u : b == 'C' ? 1u : b == 'G' ? 2u : b == 'T' ? 3u : b == 'N' ? 4u : 5u;
 }
 
+// Steps between two rebasings of the rebased form (see sw16_pair).
+constexpr int kSw16Rebase = 32;
+
 // Shared memory of one warp: the two score tables (per class and 16-byte group of 8 columns, one uint4
-// per lane), the rows' base classes (one u16 per row, X in the low byte, 32 spare rows on both sides),
-// the packed last row (per padded column) and last column (per row).
-template <int K>
+// per lane), the last row (per padded column) and last column (per row), packed, or one i32 each for X
+// and Y in the rebased form, and the rows' base classes (one u16 per row, X in the low byte, 32 spare
+// rows on both sides).
+template <int K, bool REB>
 struct Sw16Shared {
     static constexpr int NV = (K + 7) / 8;
+    static constexpr int kWords = REB ? 2 : 1;                    // per row and per column
     static constexpr uint32_t kPlane = NV * 512;                  // bytes
     static constexpr uint32_t kTable = kSw16Planes * kPlane;      // bytes, per alignment
     static constexpr uint32_t lrow_off = 2 * kTable;
-    static constexpr uint32_t lcol_off = lrow_off + 32 * K * 4;
-    PHMM_HD static uint32_t rows_off(uint32_t max_rows) { return lcol_off + ((max_rows + 4) & ~3u) * 4; }
+    static constexpr uint32_t lcol_off = lrow_off + 32 * K * 4 * kWords;
+    PHMM_HD static uint32_t rows_off(uint32_t max_rows) { return lcol_off + ((max_rows + 4) & ~3u) * 4 * kWords; }
     PHMM_HD static uint32_t bytes(uint32_t max_rows) { return (rows_off(max_rows) + (max_rows + 64) * 2 + 15) & ~15u; }
 };
 
@@ -129,36 +135,36 @@ struct Sw16Half {
     bool i32;
 };
 
-// The end cell among the cells of the last row and column that reach the maximum, visited in the
-// reference's order (anti-diagonal ascending; the last-row cell before the last-column cell).
-// H values biased, `shift` 0 for X and 16 for Y.
-__device__ inline void sw16_end_cell(const Sw16Half& h, const uint32_t* lrow, const uint32_t* lcol, int shift, int bias,
-                                     int lane, int& best, int& mi, int& mj)
+// The end cell among the cells of the last row (row(j), j = 1..ncol) and column (col(i), i = 1..nrow)
+// that reach the maximum, visited in the reference's order (anti-diagonal ascending; the last-row cell
+// before the last-column cell).
+template <typename Row, typename Col>
+__device__ inline void sw16_end_cell(int nrow, int ncol, Row row, Col col, int lane, int& best, int& mi, int& mj)
 {
-    const int nrow = h.nrow, ncol = h.ncol;
-    const uint32_t* row = lrow + h.pad - 1;  // row[j], j = 1..ncol
-    uint32_t smax = 0;
-    for (int j = 1 + lane; j <= ncol; j += 32) smax = max(smax, (row[j] >> shift) & 0xffffu);
-    for (int i = 1 + lane; i <= nrow; i += 32) smax = max(smax, (lcol[i] >> shift) & 0xffffu);
+    int smax = (int)0x80000000;
+    for (int j = 1 + lane; j <= ncol; j += 32) smax = row(j) > smax ? row(j) : smax;
+    for (int i = 1 + lane; i <= nrow; i += 32) smax = col(i) > smax ? col(i) : smax;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, o));
-    const int val = (int)smax - bias;
+    for (int o = 16; o > 0; o >>= 1) {
+        const int x = (int)__shfl_xor_sync(0xffffffffu, (uint32_t)smax, o);
+        smax = x > smax ? x : smax;
+    }
     const int alo = (nrow < ncol ? nrow : ncol) + 1, ahi = nrow + ncol;
     for (int a0 = alo; a0 <= ahi; a0 += 32) {
         const int a = a0 + lane;
-        const bool rc = a <= ahi && a >= nrow + 1 && ((row[a - nrow] >> shift) & 0xffffu) == smax;
-        const bool cc = a <= ahi && a >= ncol + 1 && ((lcol[a - ncol] >> shift) & 0xffffu) == smax;
+        const bool rc = a <= ahi && a >= nrow + 1 && row(a - nrow) == smax;
+        const bool cc = a <= ahi && a >= ncol + 1 && col(a - ncol) == smax;
         uint32_t mr = __ballot_sync(0xffffffffu, rc), mc = __ballot_sync(0xffffffffu, cc);
         while (mr | mc) {
             const int l = __ffs((int)(mr | mc)) - 1;
             const int aa = a0 + l;
             if ((mr >> l) & 1u) {
                 const int ci = nrow, cj = aa - nrow;
-                if (best < val || abs(ci - cj) < abs(mi - mj)) { best = val; mi = ci; mj = cj; }
+                if (best < smax || abs(ci - cj) < abs(mi - mj)) { best = smax; mi = ci; mj = cj; }
             }
             if ((mc >> l) & 1u) {
                 const int ci = aa - ncol, cj = ncol;
-                if (best < val || mj == ncol || abs(ci - cj) <= abs(mi - mj)) { best = val; mi = ci; mj = cj; }
+                if (best < smax || mj == ncol || abs(ci - cj) <= abs(mi - mj)) { best = smax; mi = ci; mj = cj; }
             }
             mr &= ~(1u << l);
             mc &= ~(1u << l);
@@ -174,15 +180,24 @@ __device__ inline uint32_t sw16_op(uint32_t run)
 
 // Two alignments of one class (K read columns per lane).  scr: the warp's scratch, sm: its shared
 // memory; max_rows: the launch's longest haplotype (sizes both).
-template <int K>
+//
+// REB: the rebased form, for scores beyond 16 bits (the assembly parameters).  Neighbouring H differ by
+// at most match - gap_open (down to gap_open), so what a lane holds lies within K + 1 such steps of its
+// first column, and moves by one more per row.  Each lane keeps a 32-bit base per alignment and the
+// halves hold the difference to it plus 32768; every kSw16Rebase steps all lanes move their base to their
+// first column's H.  A shuffled value is brought to the receiver's base by one add (the bases' difference,
+// exchanged at the rebasing).  Last row and column are kept as 32-bit scores.  Measured on B200, device
+// time of 2,726 haplotype-to-window alignments with the assembly parameters: 2.14 ms with one alignment
+// per warp in 32 bits, 0.91 ms here.
+template <int K, bool REB>
 __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int lane, uint8_t* scr, char* sm,
                                  uint32_t max_rows)
 {
-    using SM = Sw16Shared<K>;
+    using SM = Sw16Shared<K, REB>;
     constexpr int NV = SM::NV, NW = (K + 3) / 4, ROW = 32 * NW, S = 32 * K;
     constexpr uint32_t kSign = 0x80008000u;
     const int open = v.prm.gap_open, ext = v.prm.gap_extend, mis = v.prm.mismatch;
-    const int bias = sw16_bias(v.prm, K);
+    const int bias = REB ? 32768 : sw16_bias(v.prm, K);
     const uint32_t H0 = (uint32_t)bias * 0x10001u;
     const uint32_t LOW = (uint32_t)(bias + open - ext - 1) * 0x10001u;     // extending it stays below opening
     const uint32_t XE = (uint32_t)(-ext) * 0x10001u;
@@ -254,6 +269,26 @@ __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int 
             Fp[k] = LOW;
         }
         uint32_t hprev = H0, hout = H0, eout = LOW;
+        int base_x = 0, base_y = 0;              // REB: this lane's bases
+        uint32_t to_mine = 0, edge = 0;          // REB: from the left lane's base (lane 0: from 0) to mine
+        auto rebase = [&] {
+            const int dx = (int)(Hp[0] & 0xffffu) - 32768, dy = (int)(Hp[0] >> 16) - 32768;
+            const uint32_t d = (uint32_t)dx + ((uint32_t)dy << 16);
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                Hp[k] -= d;
+                Fp[k] -= d;
+            }
+            hprev -= d;
+            hout -= d;
+            eout -= d;
+            base_x += dx;
+            base_y += dy;
+            const uint32_t px = __shfl_up_sync(0xffffffffu, (uint32_t)base_x, 1);
+            const uint32_t py = __shfl_up_sync(0xffffffffu, (uint32_t)base_y, 1);
+            to_mine = (px - (uint32_t)base_x) + ((py - (uint32_t)base_y) << 16);
+            edge = 0u - (uint32_t)base_x - ((uint32_t)base_y << 16);
+        };
         const char* tx = sm + lane * 16;
         const char* ty = tx + SM::kTable;
         const int capX = hf[0].live ? hf[0].nrow : -1, capY = hf[1].live ? hf[1].nrow : -1;
@@ -261,11 +296,12 @@ __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int 
         auto step = [&](int t, auto full, auto raw) {
             constexpr bool FULL = decltype(full)::value, RAW = decltype(raw)::value;
             const int i = t + 1 - lane;
-            uint32_t hl = __shfl_up_sync(0xffffffffu, hout, 1);
-            uint32_t el = __shfl_up_sync(0xffffffffu, eout, 1);
+            if (REB && t % kSw16Rebase == 0 && t > 0) rebase();
+            uint32_t hl = __shfl_up_sync(0xffffffffu, hout, 1) + to_mine;
+            uint32_t el = __shfl_up_sync(0xffffffffu, eout, 1) + to_mine;
             if (lane == 0) {
-                hl = H0;
-                el = LOW;
+                hl = H0 + edge;
+                el = LOW + edge;
             }
             const uint32_t cw = rows[t - lane + 32];
             uint32_t wx[4 * NV], wy[4 * NV];
@@ -332,8 +368,24 @@ __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int 
                 uint32_t* row = bt + (uint32_t)t * ROW + lane;
 #pragma unroll
                 for (int w = 0; w < NW; ++w) row[w * 32] = code[w];
-                if (lane == 31) lcol[i] = hl;
-                if (!FULL) {
+                if (lane == 31) {
+                    if (REB) {
+                        lcol[2 * i] = (hl & 0xffffu) - 32768u + (uint32_t)base_x;
+                        lcol[2 * i + 1] = (hl >> 16) - 32768u + (uint32_t)base_y;
+                    } else {
+                        lcol[i] = hl;
+                    }
+                }
+                if (!FULL && REB) {
+                    if (i == capX) {
+#pragma unroll
+                        for (int k = 0; k < K; ++k) lrow[2 * (lane * K + k)] = (Hp[k] & 0xffffu) - 32768u + (uint32_t)base_x;
+                    }
+                    if (i == capY) {
+#pragma unroll
+                        for (int k = 0; k < K; ++k) lrow[2 * (lane * K + k) + 1] = (Hp[k] >> 16) - 32768u + (uint32_t)base_y;
+                    }
+                } else if (!FULL) {
                     if (i == capX) {
 #pragma unroll
                         for (int k = 0; k < K; ++k) ((uint16_t*)lrow)[2 * (lane * K + k)] = (uint16_t)Hp[k];
@@ -366,7 +418,13 @@ __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int 
         const Sw16Half& h = hf[q];
         bestv[q] = h.i32 ? (int)0x80000000 : -32768;
         if (h.live) {
-            sw16_end_cell(h, lrow, lcol, 16 * q, bias, lane, bestv[q], mi[q], mj[q]);
+            // row j is padded column pad + j - 1
+            auto row = [&](int j) {
+                const int c = h.pad + j - 1;
+                return REB ? (int)lrow[2 * c + q] : (int)((lrow[c] >> (16 * q)) & 0xffffu) - bias;
+            };
+            auto col = [&](int i) { return REB ? (int)lcol[2 * i + q] : (int)((lcol[i] >> (16 * q)) & 0xffffu) - bias; };
+            sw16_end_cell(h.nrow, h.ncol, row, col, lane, bestv[q], mi[q], mj[q]);
         } else {  // only boundary cells (H = 0), or no candidate at all
             if (h.nrow == 0 && h.ncol > 0) { bestv[q] = 0; mj[q] = 1; }
             if (h.ncol == 0 && h.nrow > 0) { bestv[q] = 0; mi[q] = h.nrow; }

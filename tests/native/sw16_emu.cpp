@@ -49,7 +49,6 @@ uint32_t __ballot_sync(unsigned, bool p)
 bool __any_sync(unsigned, bool p) { return __ballot_sync(0, p) != 0; }
 void __syncwarp() { t_warp->meet(); }
 int __ffs(int x) { return __builtin_ffs(x); }
-uint32_t max(uint32_t a, uint32_t b) { return a > b ? a : b; }
 }  // namespace
 
 #include "../../rovaca_b200/csrc/phmm_sw16.cuh"
@@ -75,32 +74,32 @@ struct Block {  // a zeroed, 256-byte aligned block with guard bytes on both sid
     }
 };
 
-template <int K>
+template <int K, bool REB>
 bool run(SwView v, uint32_t ix, uint32_t iy, uint32_t max_rows)
 {
-    Block scr(sw16_layout(max_rows, K).total), sm(Sw16Shared<K>::bytes(max_rows));
+    Block scr(sw16_layout(max_rows, K).total), sm(Sw16Shared<K, REB>::bytes(max_rows));
     Warp w;
     std::vector<std::thread> lanes;
     for (int l = 0; l < 32; ++l)
         lanes.emplace_back([&, l] {
             t_warp = &w;
             t_lane = l;
-            sw16_pair<K>(v, ix, iy, l, (uint8_t*)scr.p, sm.p, max_rows);
+            sw16_pair<K, REB>(v, ix, iy, l, (uint8_t*)scr.p, sm.p, max_rows);
         });
     for (auto& t : lanes) t.join();
     return scr.intact() && sm.intact();
 }
 }  // namespace
 
-// Whether width K takes these parameters (sw_packs).
-extern "C" int emu_sw16_packs(const int32_t* prm, uint32_t nrow, uint32_t ncol, int K)
+// The form (SwForm) width K runs these alignments in.
+extern "C" int emu_sw16_form(const int32_t* prm, int i32, uint32_t nrow, uint32_t ncol, int K)
 {
-    return sw_packs(SwParams{prm[0], prm[1], prm[2], prm[3]}, nrow, ncol, K);
+    return sw_form(SwParams{prm[0], prm[1], prm[2], prm[3]}, i32 != 0, nrow, ncol, K);
 }
 
-// Runs items (0, 1), or item 0 alone (n == 1); results and up to `cap` CIGAR ops per item.  0 when the
+// Runs items (0, 1), or item 0 alone (n == 1), in the plain or the rebased form; results and up to `cap` CIGAR ops per item.  0 when the
 // code stayed inside its buffers.
-extern "C" int emu_sw16(int K, const int32_t* prm, int variant, int n, const SwItem* items, const uint8_t* hap,
+extern "C" int emu_sw16(int K, int rebased, const int32_t* prm, int variant, int n, const SwItem* items, const uint8_t* hap,
                         const uint8_t* read, uint32_t cap, phmm_sw_result* out, uint32_t* ops)
 {
     SwView v{};
@@ -118,12 +117,12 @@ extern "C" int emu_sw16(int K, const int32_t* prm, int variant, int n, const SwI
     for (int q = 0; q < n; ++q) rows = rows > items[q].hap_len ? rows : items[q].hap_len;
     const uint32_t iy = n > 1 ? 1u : 0xffffffffu;
     switch (K) {
-    case 1: return !run<1>(v, 0, iy, rows);
-    case 3: return !run<3>(v, 0, iy, rows);
-    case 5: return !run<5>(v, 0, iy, rows);
-    case 8: return !run<8>(v, 0, iy, rows);
-    case 10: return !run<10>(v, 0, iy, rows);
-    case 24: return !run<24>(v, 0, iy, rows);
+    case 1: return rebased ? !run<1, true>(v, 0, iy, rows) : !run<1, false>(v, 0, iy, rows);
+    case 3: return rebased ? !run<3, true>(v, 0, iy, rows) : !run<3, false>(v, 0, iy, rows);
+    case 5: return rebased ? !run<5, true>(v, 0, iy, rows) : !run<5, false>(v, 0, iy, rows);
+    case 8: return rebased ? !run<8, true>(v, 0, iy, rows) : !run<8, false>(v, 0, iy, rows);
+    case 10: return rebased ? !run<10, true>(v, 0, iy, rows) : !run<10, false>(v, 0, iy, rows);
+    case 24: return rebased ? !run<24, true>(v, 0, iy, rows) : !run<24, false>(v, 0, iy, rows);
     default: return 2;
     }
 }

@@ -27,11 +27,14 @@ def emu():
         subprocess.run(["g++", "-O2", "-std=c++17", "-w", "-shared", "-fPIC", "-I/usr/local/cuda/include", str(SRC), "-o",
                         str(out), "-lpthread"], check=True)
     lib = C.CDLL(str(out))
-    lib.emu_sw16_packs.argtypes = [C.c_void_p, C.c_uint32, C.c_uint32, C.c_int]
+    lib.emu_sw16_form.argtypes = [C.c_void_p, C.c_int, C.c_uint32, C.c_uint32, C.c_int]
     return lib
 
 
-def _run(lib, k, params, variant, pairs):
+PLAIN, REBASED, ONE_PER_WARP = 0, 1, 2
+
+
+def _run(lib, k, rebased, params, variant, pairs):
     haps, reads = b"".join(h for h, _ in pairs), b"".join(r for _, r in pairs)
     items = np.zeros(len(pairs), sw.SW_ITEM_DTYPE)
     items["hap_len"], items["read_len"] = [len(h) for h, _ in pairs], [len(r) for _, r in pairs]
@@ -41,7 +44,7 @@ def _run(lib, k, params, variant, pairs):
     prm = (C.c_int32 * 4)(*params)
     p = lambda a: a.ctypes.data_as(C.c_void_p)
     hb, rb = np.frombuffer(haps + b"\0", np.uint8), np.frombuffer(reads + b"\0", np.uint8)
-    assert lib.emu_sw16(k, prm, variant, len(pairs), p(items), p(hb), p(rb), 2047, p(out), p(ops)) == 0
+    assert lib.emu_sw16(k, int(rebased), prm, variant, len(pairs), p(items), p(hb), p(rb), 2047, p(out), p(ops)) == 0
     return [(int(o["score"]), int(o["alignment_offset"]), int(o["max_i"]), int(o["max_j"]),
              [int(x) for x in ops[2047 * q:2047 * q + int(o["cigar_count"])]]) for q, o in enumerate(out)]
 
@@ -72,7 +75,8 @@ def test_pairs_equal_the_oracle(emu, k, alphabet):
     oracle = SwOracle()
     lo = 1 if k == 1 else 32 * (k - 1 if k <= 8 else {10: 8, 24: 20}[k])
     shapes = [(1, lo), (31, 32 * k), (40, lo + 1), (260, 32 * k), (33, 32 * k - 1), (150, lo + 7)]
-    for params, variant in ((sw.GENOTYPING, 0), ((3, -2, -5, -1), 2), ((1, 0, 0, -1), 1)):
+    for params, variant, rebased in ((sw.GENOTYPING, 0, False), ((3, -2, -5, -1), 2, False), ((1, 0, 0, -1), 1, False),
+                                     (sw.ASSEMBLY, 1, True), (sw.GENOTYPING, 0, True), ((250, 0, -200, -40), 1, True)):
         pairs = []
         for rows, cols in shapes:
             h = _sequence(rng, rows, alphabet)
@@ -82,17 +86,22 @@ def test_pairs_equal_the_oracle(emu, k, alphabet):
                   [(b"", b""), (b"A", b"A")]]
         prm = (C.c_int32 * 4)(*params)
         for g in groups:
-            assert all(emu.emu_sw16_packs(prm, len(h), len(r), k) for h, r in g)
-            assert _run(emu, k, params, variant, g) == [oracle.align(h, r, params, variant) for h, r in g], (params, g)
+            form = {emu.emu_sw16_form(prm, int(variant == 1), len(h), len(r), k) for h, r in g}
+            assert form <= ({PLAIN, REBASED} if rebased else {PLAIN})
+            assert _run(emu, k, rebased, params, variant, g) == [oracle.align(h, r, params, variant) for h, r in g], (params, g)
 
 
-def test_parameters_that_do_not_fit_16_bits_are_left_to_the_general_kernel(emu):
-    def packs(params, nrow=300, ncol=250, k=8):
-        return bool(emu.emu_sw16_packs((C.c_int32 * 4)(*params), nrow, ncol, k))
+def test_forms_of_parameters(emu):
+    def form(params, nrow=300, ncol=250, k=8, i32=True):
+        return emu.emu_sw16_form((C.c_int32 * 4)(*params), int(i32), nrow, ncol, k)
 
-    assert packs(sw.GENOTYPING) and packs(sw.GENOTYPING, 2047, 768, 24)
-    assert not packs(sw.GENOTYPING, 2048) and not packs(sw.GENOTYPING, 300, 769, 24)
-    assert not packs(sw.ASSEMBLY)                       # 256 columns x 200
-    for params in ((10, -15, 1, -5), (10, -15, -30, 0), (10, 1, -30, -5), (-1, -15, -30, -5), (10, -15, -30, -40),
-                   (200000, -15, -30, -5), (10, -15, -2**31, -5), (10, -15, -30, -2**31)):
-        assert not packs(params), params
+    assert form(sw.GENOTYPING) == form(sw.GENOTYPING, 2047, 768, 24) == form(sw.GENOTYPING, i32=False) == PLAIN
+    assert form(sw.ASSEMBLY) == form(sw.ASSEMBLY, 2047, 768, 24) == REBASED      # 256 columns x 200
+    assert form(sw.ASSEMBLY, i32=False) == REBASED
+    assert form(sw.ASSEMBLY, 300, 768, 24, i32=False) == ONE_PER_WARP            # its int16 cutoff could bind
+    for params, nrow, ncol, k in ((sw.GENOTYPING, 2048, 250, 8), (sw.GENOTYPING, 300, 769, 24),
+                                  ((10, -15, 1, -5), 300, 250, 8), ((10, -15, -30, 0), 300, 250, 8),
+                                  ((10, 1, -30, -5), 300, 250, 8), ((-1, -15, -30, -5), 300, 250, 8),
+                                  ((600, -15, -300, -5), 300, 250, 8), ((200000, -15, -30, -5), 300, 250, 8),
+                                  ((10, -15, -2**31, -5), 300, 250, 8), ((10, -15, -30, -2**31), 300, 250, 8)):
+        assert form(params, nrow, ncol, k) == ONE_PER_WARP, params
