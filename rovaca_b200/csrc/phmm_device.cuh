@@ -31,6 +31,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 
 #include "phmm_types.h"
 
@@ -113,11 +114,40 @@ struct LaneRows {
     uint32_t padmask;             // bit k: slot k is a pad row
 };
 
-// A warp's prior table: [class][row slot][lane], kTabClasses * K * kWarp values.
+// Asynchronous copies into shared memory (compiled for the host, as the CPU warp emulator does, a copy
+// completes at once).
+__device__ __forceinline__ void copy_16_async(void* dst_shared, const void* src)
+{
+#ifdef __CUDA_ARCH__
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst_shared);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+#else
+    std::memcpy(dst_shared, src, 16);
+#endif
+}
+__device__ __forceinline__ void copies_commit()
+{
+#ifdef __CUDA_ARCH__
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void copies_wait_all()
+{
+#ifdef __CUDA_ARCH__
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+#endif
+}
+
+// Columns of the FP64 kernels' ring of the row above a stripe (one (I, sum) pair per column): three
+// blocks of kScrBlock64 columns, two complete (the steps of a block and the vote's look past its end)
+// and one being copied, in four blocks of slots.
+constexpr int kScrBlock64 = 16, kScrRing64 = 4 * kScrBlock64;
+// A warp's prior table: [class][row slot][lane], kTabClasses * K * kWarp values (and, for K = 8, the only
+// multi-stripe shape, the ring of the row above).
 template <int K>
 __host__ __device__ constexpr int prior_table_size()
 {
-    return kTabClasses * K * kWarp;
+    return kTabClasses * K * kWarp + (K == kMaxK ? 2 * kScrRing64 : 0);
 }
 template <int K>
 __device__ __forceinline__ int prior_slot(uint32_t cls, int k, int lane)

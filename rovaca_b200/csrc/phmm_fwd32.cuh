@@ -40,7 +40,7 @@ template <int KH, int V, int PM, bool MULTI>
 __global__ void __launch_bounds__(kFwdBlock, min_blocks32<KH, V, PM>()) fwd_f32_kernel(BatchView b, ProbTables<float> tb,
                                                                                  PassControl pc)
 {
-    __shared__ float4 tab[tab_floats4<KH>() + kRingFloat4];
+    __shared__ float4 tab[tab_floats4<KH>() + (MULTI ? kRingFloat4 : kCodeRingFloat4)];
     const int lane = threadIdx.x & (kWarp - 1);
     const unsigned int warp_id = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
     // Over-subscribed grid (waves > 1): warps that exit after their share leave room on the SMs for
