@@ -29,7 +29,27 @@ struct LaneRowsEq {
     double xxn;                     // xx of the row below the lane (1 for a pad row)
     double mm, gm, mx;              // one value per read (mx == my)
     uint32_t padmask;               // bit k: slot k is a pad row
+    int shrink;                     // step_shrink of the lane's rows
 };
+
+__device__ __forceinline__ int larger(int a, int b) { return a > b ? a : b; }
+
+// v >= 2^-bits_below(v) for a probability v > 0; 0 for v = 0 (its products are exactly 0).
+__device__ __forceinline__ int bits_below(double v)
+{
+    return v > 0.0 ? 1023 - (int)((uint32_t)__double2hiint(v) >> 20) : 0;
+}
+
+// The bits by which one step can shrink a value at most: every nonzero result of a step, intermediate
+// ones included, is at least the smallest nonzero input times 2^-shrink.  Its longest product is M of the
+// lane's first row (prior, at least 2^-prior), carried by M * mx into the insertion chain (gap), down the
+// lane's K rows and to the row below (K factors xx, at least 2^-cont each), and into a diagonal sum (a
+// factor mm or gapm, at least 2^-keep); the last bit covers the roundings (under K + 4 of 2^-53 each).
+template <int K>
+__device__ __forceinline__ int step_shrink(int prior, int gap, int cont, int keep)
+{
+    return prior + gap + K * cont + keep + 1;
+}
 
 // Loads this lane's rows of the stripe starting at padded row first_padded_row (pad rows above the
 // read) and writes their priors to the warp's table.  Returns true when one of the lane's rows is an
@@ -53,6 +73,7 @@ __device__ __forceinline__ bool load_rows_eq(LaneRowsEq<K>& L, double* tab, cons
     const int below = first_padded_row + lane * K + K - pad;
     L.xxn = below >= 0 && below < R ? tb.ph2pr[b.read_c[roff + (uint64_t)below] & 127] : 1.0;
     L.In = L.Sn = L.Mb = L.Ib = 0.0;
+    int prior_bits = 0, cont_bits = bits_below(L.xxn);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         L.S[k] = L.Dn[k] = 0.0;
@@ -65,6 +86,8 @@ __device__ __forceinline__ bool load_rows_eq(LaneRowsEq<K>& L, double* tab, cons
             pa = tb.pmat[q];
             pb = (V == kInter) ? tb.pmis_inter[q] : tb.pmis_intra[q];
             L.xx[k] = tb.ph2pr[b.read_c[o] & 127];
+            prior_bits = larger(prior_bits, larger(bits_below(pa), bits_below(pb)));
+            cont_bits = larger(cont_bits, bits_below(L.xx[k]));
             const uint8_t base = b.read_bases[o];
             rc = match_code(base, V);
             if (V == kInter) exotic |= base_class(base) == 4u;
@@ -76,6 +99,7 @@ __device__ __forceinline__ bool load_rows_eq(LaneRowsEq<K>& L, double* tab, cons
         for (int c = 0; c < kTabClasses; ++c)
             tab[prior_slot<K>((uint32_t)c, k, lane)] = class_matches((uint32_t)c, rc, V) ? pa : pb;
     }
+    L.shrink = step_shrink<K>(prior_bits, bits_below(L.mx), cont_bits, larger(bits_below(L.mm), bits_below(L.gm)));
     return exotic;
 }
 
@@ -91,6 +115,7 @@ struct LaneRowsRow {
     double xx[K], mm[K], gm[K], mx[K], my[K];
     double xxn, mmn, gmn, mxn;      // the row below the lane (xx 1 and the rest 0 for a pad row)
     uint32_t padmask;
+    int shrink;
 };
 
 template <int K, int V>
@@ -118,6 +143,8 @@ __device__ __forceinline__ bool load_rows_row(LaneRowsRow<K>& L, double* tab, co
     };
     double myn;
     params(first_padded_row + lane * K + K - pad, L.xxn, L.mmn, L.gmn, L.mxn, myn);
+    int prior_bits = 0, cont_bits = bits_below(L.xxn), gap_bits = bits_below(L.mxn);
+    int keep_bits = larger(bits_below(L.mmn), bits_below(L.gmn));
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         L.S[k] = L.Dn[k] = 0.0;
@@ -133,13 +160,18 @@ __device__ __forceinline__ bool load_rows_row(LaneRowsRow<K>& L, double* tab, co
             const uint8_t base = b.read_bases[o];
             rc = match_code(base, V);
             if (V == kInter) exotic |= base_class(base) == 4u;
+            prior_bits = larger(prior_bits, larger(bits_below(pa), bits_below(pb)));
         } else {
             L.padmask |= 1u << k;
         }
+        cont_bits = larger(cont_bits, bits_below(L.xx[k]));
+        gap_bits = larger(gap_bits, larger(bits_below(L.mx[k]), bits_below(L.my[k])));
+        keep_bits = larger(keep_bits, larger(bits_below(L.mm[k]), bits_below(L.gm[k])));
 #pragma unroll
         for (int c = 0; c < kTabClasses; ++c)
             tab[prior_slot<K>((uint32_t)c, k, lane)] = class_matches((uint32_t)c, rc, V) ? pa : pb;
     }
+    L.shrink = step_shrink<K>(prior_bits, gap_bits, cont_bits, keep_bits);
     return exotic;
 }
 
@@ -222,14 +254,12 @@ __device__ __forceinline__ double row_diag(const LaneRowsRow<K>& L, int k, doubl
     return diag_eq<V, true>(L.gm[k], L.mm[k], dgM, dgI, dgD);
 }
 
-// Whether every nonzero input of the lane's next STEPS steps reaches flush_free_hi<K, STEPS>(): its rows' pending sums and next-column D, and the two values it hands the lane
-// below (that lane's first-row inputs).  The longest product chain of a step is still K + 1 factors
-// (the insertion chain from the first row's M down to the value handed on), so the bound of
-// rows_flush_free holds.
-// The minimum is taken as a tree (depth log2(2 K + 2) instead of a chain of 2 K + 2 dependent
-// operations): the next step's arithmetic waits on this vote.
-template <int K, int STEPS, typename LR>
-__device__ __forceinline__ bool rows_flush_free_eq(const LR& L)
+// The smallest nonzero value among the inputs of the lane's next step, by its high word less 1 (a zero
+// wraps to the largest): its rows' pending sums and next-column D, and the two values it hands the lane
+// below (that lane's first-row inputs).  Flushed values are 0 or normal, so a zero high word means 0.
+// Taken as a tree (depth log2(2 K + 2) instead of a chain of 2 K + 2 dependent operations).
+template <int K, typename LR>
+__device__ __forceinline__ uint32_t rows_min_hi(const LR& L)
 {
     constexpr int N = 2 * K + 2;
     uint32_t v[N];
@@ -245,13 +275,13 @@ __device__ __forceinline__ bool rows_flush_free_eq(const LR& L)
 #pragma unroll
         for (int i = 0; i + w < N; i += 2 * w) v[i] = min(v[i], v[i + w]);
     }
-    return v[0] >= flush_free_hi<K, STEPS>() - 1u;
+    return v[0];
 }
 
 // Sweep one stripe over the column stream of haplotypes [g_lo, g_hi): as `sweep` (phmm_device.cuh),
 // the scratch row holding the handed-on (I, sum) pair per column.  LR: LaneRowsEq or LaneRowsRow.
 template <int K, int V, bool FROM_SCR, bool TO_SCR, typename LR>
-__device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const ProbTables<double>& tb,
+__device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTables<double>& tb,
                          const SweepOut& so, uint32_t g_lo, uint32_t g_hi, double* scr, int lane, bool above_row0,
                          bool exotic, uint64_t roff, int R, int row0)
 {
@@ -266,14 +296,42 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
     double D0 = 0.0;
     double Stop = 0.0;  // lane 0's first-row sum below the boundary row (M = I = 0, D = C/H)
     double sumM = 0.0, sumI = 0.0;
-    // flush_free: the current two steps' inputs are all 0 or above the bound.  The vote for the next two
-    // is taken after the first of these, on the bound of three steps, so that the second step's
-    // arithmetic covers its latency (the branch below waits on it): 26.5 against 27.6 ms for the FP64
-    // pass of 60 underflow-stress regions with a vote after every second step and a branch per step.
+    // Steps run in chunks of four, with the flushes of every result or, when the vote has shown that no
+    // result of the chunk can fall below 2^-1022, without.  The vote is taken in the middle of the chunk
+    // before, so that the steps behind it cover its latency (the chunk's branch waits on it), on the bound
+    // of the six steps up to the chunk's end.  The bound follows from the item's own probabilities
+    // (step_shrink): about 65 bits a step for 8 rows a lane and qualities up to 45, where the smallest
+    // probability of any quality would give 396.  Measured on B200, FP64 pass of 60 low-quality regions:
+    // 26.1 ms with a vote per two steps on that smallest-probability bound, 25.1 ms so.
     bool flush_free = false, free_next = false;
-    uint32_t wn = codes[-lane];  // the code word of the lane's next column, loaded a step ahead (26.1 ms)
+    uint32_t wn = codes[-lane];  // the code word of the lane's next column, loaded a step ahead
+
+    int shrink = L.shrink;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) shrink = larger(shrink, __shfl_sync(0xffffffffu, shrink, lane ^ o));
+    constexpr int kAhead = kChunkScalar / 2 + kChunkScalar;  // steps a vote covers
+    const uint32_t free_hi = 1 + kAhead * shrink < 2046 ? ((uint32_t)(1 + kAhead * shrink) << 20) - 1u : 0xffffffffu;
 
     const int steps = Tcols + kWarp;
+    // Stripes after the first: the row above (scratch, one 16-byte pair per column) comes through a ring
+    // in shared memory, copied two blocks ahead, so that lane 0 does not wait for L2 in every step and
+    // the vote can look at the values the next steps will take (FP64 pass of 24 regions of long reads 6.6
+    // and 6.2 ms; far from a read's alignment there are always values near 2^-1022, so most steps of long
+    // reads keep their flushes).  Lane 31 writes the same row 31 columns
+    // behind lane 0 (for the stripe below), never a column still to be read.
+    static_assert(!FROM_SCR || K == kMaxK, "the ring is part of the multi-stripe shape's table");
+    double* ring = tab + kTabClasses * K * kWarp;
+    auto copy_block = [&](int c0) {
+        if (lane < kScrBlock64 && c0 + lane < Tcols) {
+            const int c = c0 + lane;
+            copy_16_async(&ring[2 * (c & (kScrRing64 - 1))], scr + 2 * c);
+        }
+        copies_commit();
+    };
+    if (FROM_SCR) {
+        copy_block(0);
+        copy_block(kScrBlock64);
+    }
 
     auto boundary = [&]() {
         if (started) {
@@ -310,7 +368,7 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
         }
     };
 
-    constexpr bool kVote = PHMM_F64_VOTE && !FROM_SCR;
+    constexpr bool kVote = PHMM_F64_VOTE;
     auto step = [&](int t, bool check, auto flush) {
         constexpr bool FL = decltype(flush)::value;
         const int p = t - lane;
@@ -320,8 +378,8 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
         if (lane == 0) {
             if (FROM_SCR) {
                 const bool ok = p >= 0 && p < Tcols;
-                uI = ok ? scr[2 * p + 0] : 0.0;
-                uS = ok ? scr[2 * p + 1] : 0.0;
+                uI = ok ? ring[2 * (p & (kScrRing64 - 1)) + 0] : 0.0;
+                uS = ok ? ring[2 * (p & (kScrRing64 - 1)) + 1] : 0.0;
             } else {
                 // below the boundary row: I = fma(0, xx, 0 * mx) = 0
                 uI = 0.0;
@@ -353,26 +411,37 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
             sumI = radd(sumI, L.Ib);
         }
         if constexpr (kVote) {
-            if (t % 2 == 0) free_next = __all_sync(0xffffffffu, rows_flush_free_eq<K, 3>(L));
-            else flush_free = free_next;
+            if (t % kChunkScalar == kChunkScalar / 2 - 1) {
+                uint32_t v = rows_min_hi<K>(L);
+                if (FROM_SCR && lane < kAhead && t + 1 + lane < Tcols) {  // lane 0's inputs of the covered steps
+                    const double* q = ring + 2 * ((t + 1 + lane) & (kScrRing64 - 1));
+                    v = min(v, min((uint32_t)__double2hiint(q[0]) - 1u, (uint32_t)__double2hiint(q[1]) - 1u));
+                }
+                free_next = __all_sync(0xffffffffu, v >= free_hi);
+            } else if (t % kChunkScalar == kChunkScalar - 1) {
+                flush_free = free_next;
+            }
         }
     };
-    static_assert(kChunkScalar % 2 == 0, "steps run in pairs");
+    static_assert(kChunkScalar % 2 == 0 && kScrBlock64 % kChunkScalar == 0 && kAhead <= kScrBlock64 && kAhead <= kWarp,
+                  "a vote looks at most one block ahead");
     const auto yes = std::true_type{};
     const auto no = std::false_type{};
 
     for (int t0 = 0; t0 < steps; t0 += kChunkScalar) {
+        if (FROM_SCR && t0 % kScrBlock64 == 0) {  // columns up to t0 + 2 blocks are complete from here
+            copies_wait_all();
+            __syncwarp();
+            copy_block(t0 + 2 * kScrBlock64);
+        }
         const int nb31 = __shfl_sync(0xffffffffu, nb, kWarp - 1);
         if (nb31 >= t0 + kChunkScalar && t0 + kChunkScalar <= steps) {
+            if (kVote && flush_free) {
 #pragma unroll
-            for (int u = 0; u < kChunkScalar; u += 2) {
-                if (kVote && flush_free) {
-                    step(t0 + u, false, no);
-                    step(t0 + u + 1, false, no);
-                } else {
-                    step(t0 + u, false, yes);
-                    step(t0 + u + 1, false, yes);
-                }
+                for (int u = 0; u < kChunkScalar; ++u) step(t0 + u, false, no);
+            } else {
+#pragma unroll
+                for (int u = 0; u < kChunkScalar; ++u) step(t0 + u, false, yes);
             }
         } else {
             for (int u = 0; u < kChunkScalar; ++u)
@@ -381,6 +450,10 @@ __device__ void sweep_eq(LR& L, const double* tab, const BatchView& b, const Pro
                     else step(t0 + u, true, yes);
                 }
         }
+    }
+    if (FROM_SCR) {
+        copies_wait_all();
+        __syncwarp();
     }
 }
 

@@ -44,7 +44,7 @@ __device__ __forceinline__ void run_read(const BatchView& b, const ProbTables<T>
                 exotic = load_rows_row<K, V>(L, tab, b, tb, roff, R, s * SR, pad, lane);
             const bool above_row0 = (s == 0) && (lane * K <= pad);
             const int row0 = s * SR - pad;  // read position of slot 0 of lane 0
-            if (!MULTI)
+            if constexpr (!MULTI)
                 sweep_eq<K, V, false, false>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R, row0);
             else if (s == 0)
                 sweep_eq<K, V, false, true>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R, row0);
