@@ -36,47 +36,82 @@ __constant__ uint8_t c_pcr_caps[4][21] = {
     {40, 40, 40, 40, 39, 39, 39, 39, 39, 38, 38, 38, 37, 37, 37, 36, 36, 35, 34, 33, 33},  // CONSERVATIVE
 };
 
-// Copies of s[u, u+ul) tiling s[t, t+tl) from its front (leading) or back, stopping at the first
-// copy that differs; counting stops at 21, which is enough because the repeat length is capped at 20
-// and the search only asks whether a count exceeds 1.
-__device__ int count_repeats(const uint8_t* s, int n, int u, int ul, int t, int tl, bool leading)
+constexpr int kMaxUnit = 8;                          // longest repeat unit
+constexpr int kEqWords = (kMaxReadLen + 31) / 32 + 1;  // words of a read's equality mask, and one of zeros
+
+// Equality masks of one read: bit i of eq[u - 1] is set when base i equals base i + u (i + u inside the
+// read).  A unit of u bases repeats as long as its mask stays set, so repeats are counted as runs of
+// ones.  Built by the whole warp.
+__device__ __forceinline__ void build_equal(uint32_t (*eq)[kEqWords], const uint8_t* s, int n, int lane)
 {
-    if (tl <= 0 || ul <= 0 || ul > tl || u < 0 || t < 0 || u + ul > n || t + tl > n) return 0;
-    int k = 0;
-    for (int c = 0; c < tl / ul && k < 21; ++c) {
-        const int start = leading ? c * ul : tl - (c + 1) * ul;
-        bool same = true;
-        for (int x = 0; x < ul; ++x) same &= s[t + start + x] == s[u + x];
-        if (!same) break;
-        ++k;
+    const int words = (n + 31) / 32;
+    for (int w = 0; w <= words; ++w) {
+        const int i = w * 32 + lane;
+        const uint8_t c = i < n ? s[i] : 0;
+#pragma unroll
+        for (int u = 1; u <= kMaxUnit; ++u) {
+            const uint32_t m = __ballot_sync(0xffffffffu, i + u < n && s[i + u] == c);
+            if (lane == u - 1) eq[u - 1][w] = m;
+        }
     }
-    return k;
+}
+
+// Ones of mask m from bit i upwards.  (A read's last word, or the word of zeros after it, ends the run.)
+__device__ __forceinline__ int ones_from(const uint32_t* m, int i)
+{
+    int run = 0;
+    for (;;) {
+        const int b = i & 31;
+        const uint32_t x = ~m[i >> 5] >> b;         // zeros of m from bit i on
+        if (x) return run + __ffs((int)x) - 1;
+        run += 32 - b;
+        i += 32 - b;
+    }
+}
+
+// Ones of mask m from bit i downwards.
+__device__ __forceinline__ int ones_down(const uint32_t* m, int i)
+{
+    int run = 0;
+    while (i >= 0) {
+        const int b = i & 31;
+        const int k = __clz((int)~(m[i >> 5] << (31 - b)));  // at most b + 1 ones
+        run += k;
+        if (k <= b) break;
+        i -= k;
+    }
+    return run;
 }
 
 // Tandem-repeat length around position o < n - 1: the shortest unit (<= 8) starting at o + 1 that
 // repeats at least twice forwards (else the single base at o + 1), its forward copies from o + 1
 // plus its copies ending at o, capped at 20.
-__device__ int repeat_length(const uint8_t* s, int n, int o)
+__device__ int repeat_length(const uint32_t (*eq)[kEqWords], int n, int o)
 {
-    int fw_str = 1, max_fw = 0;
-    for (int str = 1; str <= 8; ++str) {
-        if (o + str + 1 > n) break;
-        max_fw = count_repeats(s, n, o + 1, str, o + 1, n - o - 1, true);
-        if (max_fw > 1) {
-            fw_str = str;
+    int unit = 1, copies = 1;
+    const int w = (o + 1) >> 5, b = (o + 1) & 31;
+    for (int u = 1; u <= kMaxUnit && o + u + 1 <= n; ++u) {
+        const uint32_t next = __funnelshift_r(eq[u - 1][w], eq[u - 1][w + 1], b);  // bits o + 1 ..
+        if ((~next & ((1u << u) - 1u)) == 0u) {  // u equal bases: a second copy follows
+            unit = u;
+            copies = 1 + ones_from(eq[u - 1], o + 1) / u;
             break;
         }
     }
-    const int max_bw = count_repeats(s, n, o + 1, fw_str, 0, o + 1, false);
-    const int rl = max_bw + max_fw;
+    const int rl = copies + ones_down(eq[unit - 1], o) / unit;
     return rl > 20 ? 20 : rl;
 }
 
-// One warp per read of a region-API region: the read's bases are staged in shared memory and each
-// lane prepares positions lane, lane + 32, ...
+// Blocks (x, y): the regions x, x + gridDim.x, ..., of which block row y takes every gridDim.y-th group
+// of kPrepWarps reads, one warp per read: the read's bases are staged in shared memory, its equality
+// masks built once, and each lane prepares positions lane, lane + 32, ....
+// Latency-bound for one region (one block of 8 warps took a 40-read region's PCR model in five rounds of
+// byte-wise repeat searches).  Measured on B200, a call_pairhmm of 40 reads of 150 bases: device time
+// 187 us with that, 97 us so.
 __global__ void __launch_bounds__(kPrepWarps * 32) read_prep_kernel(RegionApiView v)
 {
     __shared__ uint8_t bases[kPrepWarps][kMaxReadLen];
+    __shared__ uint32_t equal[kPrepWarps][kMaxUnit][kEqWords];
     const BatchDesc* d = v.desc;
     if (d->region_api == 0) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -85,21 +120,26 @@ __global__ void __launch_bounds__(kPrepWarps * 32) read_prep_kernel(RegionApiVie
         const RegionDesc rg = v.regions[g];
         if (!(rg.api & kRegionApi)) continue;
         const int pcr = (rg.api >> 8) & 0xff;
-        for (uint32_t k = w; k < rg.n_reads; k += kPrepWarps) {
+        const bool capped = pcr >= 1 && pcr <= 3;
+        for (uint32_t k = blockIdx.y * kPrepWarps + w; k < rg.n_reads; k += gridDim.y * kPrepWarps) {
             const uint32_t r = rg.read_begin + k;
             const uint64_t a = v.read_off[r];
             const int n = (int)(v.read_off[r + 1] - a);
             if (n <= 0 || n > kMaxReadLen) continue;  // lengths are validated on the host
-            for (int i = lane; i < n; i += 32) bases[w][i] = v.read_bases[a + i];
-            __syncwarp();
+            if (capped) {
+                for (int i = lane; i < n; i += 32) bases[w][i] = v.read_bases[a + i];
+                __syncwarp();
+                build_equal(equal[w], bases[w], n, lane);
+                __syncwarp();
+            }
             const uint8_t mq = v.mapq[r];
             for (int i = lane; i < n; i += 32) {
                 const uint8_t q0 = v.read_q[a + i];
                 const uint8_t q = q0 < mq ? q0 : mq;
                 v.read_q[a + i] = (int)q < rg.min_quality ? (uint8_t)6 : q;
                 uint8_t gop = 45;
-                if (pcr >= 1 && pcr <= 3 && i < n - 1) {
-                    const uint8_t cap = c_pcr_caps[pcr][repeat_length(bases[w], n, i)];
+                if (capped && i < n - 1) {
+                    const uint8_t cap = c_pcr_caps[pcr][repeat_length(equal[w], n, i)];
                     if (gop >= cap) gop = cap;
                 }
                 v.read_i[a + i] = gop;
@@ -202,7 +242,9 @@ __device__ __forceinline__ double approx_log10sum(double a, double b, const doub
 // genotype g = (a <= b), g = b(b+1)/2 + a, gets
 //   GL = sum_r v_r - K log10(2),  v_r = lk(r,a) + log10(2) if a == b else log10sum(lk(r,a), lk(r,b)),
 // summed from 0 in read order (GenotypeLikelihoodCalculator, genotype_likelihood_calculator.cpp:
-// 59-100 and .h:90-142).  The most likely genotype is the first maximum.
+// 59-100 and .h:90-142): a warp per genotype, its lanes forming the terms of 32 reads at a time (the
+// loads and the table look-up of a term take most of a microsecond, the additions are in order).  The most
+// likely genotype is the first maximum.
 __global__ void __launch_bounds__(kPostThreads) genotype_kernel(RegionApiView v)
 {
     const BatchDesc* d = v.desc;
@@ -235,17 +277,22 @@ __global__ void __launch_bounds__(kPostThreads) genotype_kernel(RegionApiView v)
         __syncthreads();
         const uint32_t G = A * (A + 1) / 2;
         double* gl = v.gl + ev.gl_off;
-        for (uint32_t g = threadIdx.x; g < G; g += blockDim.x) {
+        for (uint32_t g = threadIdx.x >> 5; g < G; g += blockDim.x >> 5) {
             uint32_t b = 0;
             while ((b + 1) * (b + 2) / 2 <= g) ++b;
             const uint32_t a = g - b * (b + 1) / 2;
             const double* la = alk + (uint64_t)a * N;
             const double* lb = alk + (uint64_t)b * N;
             double sum = 0.0;
-            for (uint32_t r = 0; r < K; ++r)
-                sum = __dadd_rn(sum, a == b ? __dadd_rn(la[r], v.log10_two) : approx_log10sum(la[r], lb[r], v.jacobian));
+            for (uint32_t r0 = 0; r0 < K; r0 += 32) {
+                const uint32_t r = r0 + (threadIdx.x & 31);
+                double term = 0.0;
+                if (r < K) term = a == b ? __dadd_rn(la[r], v.log10_two) : approx_log10sum(la[r], lb[r], v.jacobian);
+                const uint32_t m = K - r0 < 32 ? K - r0 : 32;
+                for (uint32_t k = 0; k < m; ++k) sum = __dadd_rn(sum, __shfl_sync(0xffffffffu, term, k));
+            }
             // explicit roundings: no fused multiply-add, as the host computes it
-            gl[g] = __dsub_rn(sum, __dmul_rn((double)K, v.log10_two));
+            if ((threadIdx.x & 31) == 0) gl[g] = __dsub_rn(sum, __dmul_rn((double)K, v.log10_two));
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -268,7 +315,7 @@ cudaError_t launch_genotype(const RegionApiView& v, int num_sms, cudaStream_t st
 
 cudaError_t launch_read_prep(const RegionApiView& v, int num_sms, cudaStream_t st)
 {
-    read_prep_kernel<<<num_sms * 4, kPrepWarps * 32, 0, st>>>(v);
+    read_prep_kernel<<<dim3(num_sms, 4), kPrepWarps * 32, 0, st>>>(v);
     return cudaGetLastError();
 }
 

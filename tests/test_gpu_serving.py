@@ -273,6 +273,25 @@ def test_device_region_path_equals_host_preparation(engine, pcr):
         assert 0 < keep.sum() < len(reads)
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 127, 767, 768])
+def test_repeat_caps_at_mask_word_edges(engine, n):
+    """The PCR caps of reads that are one repeat from end to end (units of 1 to 9 bases, and of the read's
+    own length), at read lengths around the 32-base words of the device's equality masks: the host
+    functions' results."""
+    rng = np.random.default_rng(n)
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    reads = []
+    for unit in (1, 2, 3, 5, 8, 9, n):
+        u = bytes(acgt[rng.integers(0, 4, unit)])
+        reads.append((u * (n // unit + 1))[:n])
+    haps = [reads[1] + b"ACGTACGT", (reads[4] + reads[2])[:1536]]
+    quals = [rng.integers(10, 42, n).astype(np.uint8).tobytes() for _ in reads]
+    mapq = np.full(len(reads), 60, np.uint8)
+    got, keep = engine.call_region(haps, reads, quals, mapq, 18, 3)
+    want, wkeep = _host_region_path(engine, haps, reads, quals, mapq, 18, 3)
+    assert np.array_equal(keep, wkeep) and np.array_equal(got, want, equal_nan=True)
+
+
 def test_region_and_plain_requests_mix(engine):
     """Region-API and plain requests submitted together from several threads: each gets the result
     it gets alone (the loop batches each kind separately)."""
