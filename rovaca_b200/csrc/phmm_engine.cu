@@ -1,15 +1,16 @@
 // PairHMM engine runtime (see phmm_engine.h).
 //
 // Device arena layout (one cudaMalloc per slot, 256-byte aligned sections):
-//   descriptor block  BatchDesc | ClassDesc x 18 | status words     (one H2D copy per batch)
-//   plan arrays       regions, read_off, hap_off, read/hap N flags, work items
-//   read data         bases, q, ins, del, gcp (1 byte per base each)
-//   haplotypes        bases, then two u32 match-code streams with guard codes on both ends
-//   region API        MAPQ and kept flag per read, kept count per region
-//   results           likelihoods (f64), pair flags (u8), normalised likelihoods (f64, region API),
-//                     FP64 rerun slots (16 B per pair)
-//   scratch           per-warp stripe row for reads longer than 256 (3 values per column)
-// The arena only grows; all kernel arguments are arena pointers, so a graph captured for an arena
+//   inputs            regions, read_off, hap_off, read/hap N flags, work items, events, MAPQ, read
+//                     bases and qualities (1 byte per base each), haplotype bases
+//   descriptor block  BatchDesc | ClassDesc x 66 | status words
+//   results           region API: kept count per region, kept flag per read, genotypes; likelihoods
+//                     (f64), pair flags (u8)
+//   working data      two u32 haplotype code streams with guard codes on both ends, the likelihoods
+//                     before post-processing (region API), FP64 rerun slots (24 B per pair), per-warp
+//                     stripe rows for reads longer than 256 (3 values per column)
+// A small batch uses the same order at its own sizes, so that its inputs and its results are one piece
+// each (kCompactBytes).  The arena only grows; all kernel arguments are arena pointers, so a graph captured for an arena
 // replays for every batch that fits it.
 #include "phmm_engine.h"
 #include "phmm_sw.h"
@@ -59,8 +60,23 @@ constexpr uint64_t kDefaultChunkCells = 40000000000ull;
 // the graph leaves the host free.
 constexpr uint64_t kDirectCells = 20000000000ull;
 
-// Carves the arena for capacity c starting at base (nullptr: only measure).  Returns the size.
-size_t carve(const Capacity& c, char* base, Slot* s)
+// A batch whose inputs and whose results each take at most this much is laid out compactly, in the
+// arena's first bytes: its inputs go up in one copy from the pinned staging and its results come back in
+// one, instead of 12 to 16 copies up and 2 to 6 back of about 2.5 us of host time and 2 us of stream time
+// each.  Measured on B200, end to end: call_pairhmm on 40 reads 242 and 175 us, schedule_pairhmm on 250
+// reads 590 and 537 us.  Larger batches keep fixed sections (their graph's pointers) and copy their bases
+// straight from the caller's buffers while the host plans.
+constexpr size_t kCompactBytes = 1u << 20;
+
+// Byte ranges of a carved arena that travel together: everything the host sends, and everything it reads
+// back (they overlap in the descriptor block, which ends the first and starts the second).
+struct Spans {
+    size_t in_end = 0, out_begin = 0, out_end = 0;
+};
+
+// Carves the arena for capacity c starting at base (nullptr: only measure).  Returns the size.  api: the
+// gap qualities are written on the device and the post-processed likelihoods are the result.
+size_t carve(const Capacity& c, char* base, Slot* s, bool api = false, Spans* spans = nullptr)
 {
     size_t o = 0;
     auto take = [&](size_t bytes) -> char* {
@@ -68,33 +84,41 @@ size_t carve(const Capacity& c, char* base, Slot* s)
         o = align_up(o + std::max<size_t>(bytes, 1));
         return base ? base + at : nullptr;
     };
-    char* desc = take(kDescBytes);
-    char* desc_pristine = take(kDescBytes);
+    char *ri = nullptr, *rd = nullptr, *rc = nullptr, *out = nullptr, *out2 = nullptr;
+    auto gaps = [&] {
+        ri = take(c.read_bases);
+        rd = take(c.read_bases);
+        rc = take(c.read_bases);
+    };
     char* regions = take(c.regions * sizeof(RegionDesc));
     char* read_off = take((c.reads + 1) * sizeof(uint64_t));
     char* hap_off = take((c.haps + 1) * sizeof(uint64_t));
     char* read_flags = take(c.reads);
     char* hap_flags = take(c.haps);
     char* items = take(c.items * sizeof(WorkItem));
-    char* rb = take(c.read_bases);
-    char* rq = take(c.read_bases);
-    char* ri = take(c.read_bases);
-    char* rd = take(c.read_bases);
-    char* rc = take(c.read_bases);
-    char* hb = take(c.hap_bases);
-    char* mapq = take(c.reads);
-    char* keep = take(c.reads);
-    char* nkept = take(c.regions * sizeof(uint32_t));
-    char* ci = take((c.hap_bases + 2 * kCodePad) * sizeof(uint32_t));
-    char* ca = take((c.hap_bases + 2 * kCodePad) * sizeof(uint32_t));
-    char* out = take(c.out * sizeof(double));
-    char* pf = take(c.out);
-    char* out2 = take(c.out * sizeof(double));
     char* events = take(c.events * sizeof(EventDesc));
     char* hap_allele = take(c.hap_allele);
-    char* allele_lk = take(c.allele_lk * sizeof(double));
-    char* gl = take(c.gl * sizeof(double));
+    char* mapq = take(c.reads);
+    char* rb = take(c.read_bases);
+    char* rq = take(c.read_bases);
+    if (!api) gaps();
+    char* hb = take(c.hap_bases);
+    const size_t desc_at = o;
+    char* desc = take(kDescBytes);
+    const size_t in_end = o;
+    char* nkept = take(c.regions * sizeof(uint32_t));
+    char* keep = take(c.reads);
     char* best = take(c.events * sizeof(int32_t));
+    char* gl = take(c.gl * sizeof(double));
+    (api ? out2 : out) = take(c.out * sizeof(double));
+    char* pf = take(c.out);
+    if (spans) *spans = Spans{in_end, desc_at, o};
+    char* desc_pristine = take(kDescBytes);
+    if (api) gaps();
+    char* ci = take((c.hap_bases + 2 * kCodePad) * sizeof(uint32_t));
+    char* ca = take((c.hap_bases + 2 * kCodePad) * sizeof(uint32_t));
+    (api ? out : out2) = take(c.out * sizeof(double));
+    char* allele_lk = take(c.allele_lk * sizeof(double));
     char* rerun = take(c.rerun * sizeof(RerunEntry));
     char* scratch = take(c.scratch_cols * 3 * sizeof(double));  // c.scratch_cols counts all warps' columns
     if (s) {
@@ -138,7 +162,7 @@ size_t pinned_bytes_for(const Capacity& c)
 {
     return align_up(kDescBytes) + align_up(c.regions * sizeof(RegionDesc)) + align_up((c.reads + 1) * 8) +
            align_up((c.haps + 1) * 8) + align_up(c.reads) + align_up(c.haps) + align_up(c.items * sizeof(WorkItem)) +
-           align_up(c.events * sizeof(EventDesc)) + align_up(c.hap_allele);
+           align_up(c.events * sizeof(EventDesc)) + align_up(c.hap_allele) + 2 * kCompactBytes;
 }
 
 Capacity need_of(const Plan& p, uint64_t scratch_warps)
@@ -587,6 +611,7 @@ phmm_status Engine::reserve(Slot& s, const Capacity& want, std::string& err)
     }
     s.dev_bytes = bytes;
     carve(nc, s.dev, &s);
+    s.compact = false;
     const size_t pb = pinned_bytes_for(nc);
     e = cudaMallocHost((void**)&s.pinned, pb);
     if (e != cudaSuccess) {
@@ -692,7 +717,7 @@ phmm_status Engine::launch_pipeline(Slot& s, bool want_flags, const Plan* plan, 
     s.launches = 0;
     PHMM_CK(cudaEventRecordWithFlags(s.ev_t0, s.main, rec));
     PHMM_CK(launch_prep(s.d_desc, s.d_hb, s.d_codes_inter, s.d_codes_intra, s.d_out, v.pair_flags, sms_, s.main));
-    s.launches += 2;
+    ++s.launches;
     const RegionApiView rv = region_view(s, d_jacobian_, log10_two_);
     if (!plan || plan->region_api) {
         PHMM_CK(launch_read_prep(rv, sms_, s.main));
@@ -709,8 +734,10 @@ phmm_status Engine::launch_pipeline(Slot& s, bool want_flags, const Plan* plan, 
         const int n_cls = pass == 0 ? kClasses32 : kClasses64;
         const int slot0 = pass == 0 ? 0 : kClasses32;  // descriptor slot of the pass's first class
         for (int k = 0; k < n_cls; ++k) {
-            // FP32 classes of a mode longest reads first (multi-stripe shapes, then KH = 8 .. 1)
-            const int c = pass == 0 && s.overlap ? (k / kShapes32) * kShapes32 + kShapes32 - 1 - k % kShapes32 : k;
+            // direct launches and serving slots: the classes of a mode longest reads first (multi-stripe
+            // shapes, then KH or K = 8 .. 1), so that the longest kernels start first
+            const int per = pass == 0 ? kShapes32 : 9;
+            const int c = plan || (pass == 0 && s.overlap) ? (k / per) * per + per - 1 - k % per : k;
             uint32_t work = 0;
             if (plan) {
                 work = pass == 0 ? plan->classes[c].n_items : plan->classes[slot0 + c].rerun_cap;
@@ -800,8 +827,17 @@ phmm_status Engine::capture_graph(Slot& s, bool want_flags, const TileTable& til
     return PHMM_OK;
 }
 
+void Engine::full_layout(Slot& s)
+{
+    if (s.compact) carve(s.cap, s.dev, &s);
+    s.compact = false;
+}
+
 bool Engine::upload_raw(Slot& s, const BatchScan& sc, const phmm_batch& b)
 {
+    // (a batch that may fit the compact layout waits for its plan)
+    if (sc.cells < kDirectCells && 5 * sc.read_bases + sc.hap_bases <= kCompactBytes / 2) return false;
+    if (s.dev) full_layout(s);
     if (!s.dev || sc.read_bases > s.cap.read_bases || sc.hap_bases > s.cap.hap_bases) return false;
     cudaStream_t m = s.main;
     const uint64_t rb = sc.read_bases;
@@ -823,7 +859,7 @@ bool Engine::upload_raw(Slot& s, const BatchScan& sc, const phmm_batch& b)
 }
 
 phmm_status Engine::upload(Slot& s, const Plan& plan, const phmm_batch& b, std::string& err, const uint8_t* mapq,
-                           bool raw_sent)
+                           bool raw_sent, bool may_compact)
 {
     if (plan.region_api && plan.n_reads && !mapq) {
         err = "region-API batch without MAPQ";
@@ -834,15 +870,6 @@ phmm_status Engine::upload(Slot& s, const Plan& plan, const phmm_batch& b, std::
     if (st != PHMM_OK) return st;
     if (s.arena_grows != grows) raw_sent = false;  // a new arena: copies into the old one are gone
     PHMM_CK(cudaSetDevice(dev_));
-    // stage descriptors + plan arrays in pinned memory, then copy
-    char* p = s.pinned;
-    size_t o = 0;
-    auto stage = [&](const void* src, size_t bytes) -> char* {
-        char* at = p + o;
-        if (bytes) std::memcpy(at, src, bytes);
-        o = align_up(o + std::max<size_t>(bytes, 1));
-        return at;
-    };
     BatchDesc bd{};
     bd.hap_bases_total = plan.hap_bases;
     bd.out_total = plan.out_total;
@@ -853,10 +880,57 @@ phmm_status Engine::upload(Slot& s, const Plan& plan, const phmm_batch& b, std::
     bd.read_bases_total = plan.read_bases;
     bd.region_api = plan.region_api ? plan.n_regions : 0;
     bd.n_events = (uint32_t)plan.events.size();
+    auto put_desc = [&](char* desc) {
+        std::memcpy(desc, &bd, sizeof(bd));
+        std::memcpy(desc + sizeof(bd), plan.classes.data(), sizeof(ClassDesc) * kNumClasses);
+        std::memset(desc + sizeof(bd) + sizeof(ClassDesc) * kNumClasses, 0, 4 * sizeof(unsigned int));
+    };
+    if (may_compact && !raw_sent && !use_graph(plan)) {
+        const Capacity need = need_of(plan, scratch_warps());
+        Spans sp;
+        carve(need, nullptr, nullptr, plan.region_api, &sp);
+        if (sp.in_end <= kCompactBytes && sp.out_end - sp.out_begin <= kCompactBytes) {
+            carve(need, s.dev, &s, plan.region_api);
+            s.compact = true;
+            s.out_begin = sp.out_begin;
+            s.out_bytes = sp.out_end - sp.out_begin;
+            auto put = [&](const void* dst, const void* src, size_t bytes) {
+                if (bytes) std::memcpy(s.pinned + ((const char*)dst - s.dev), src, bytes);
+            };
+            put(s.d_regions, plan.regions.data(), plan.regions.size() * sizeof(RegionDesc));
+            put(s.d_read_off, plan.read_off.data(), plan.read_off.size() * 8);
+            put(s.d_hap_off, plan.hap_off.data(), plan.hap_off.size() * 8);
+            put(s.d_read_flags, plan.read_flags.data(), plan.read_flags.size());
+            put(s.d_hap_flags, plan.hap_flags.data(), plan.hap_flags.size());
+            put(s.d_items, plan.items.data(), plan.items.size() * sizeof(WorkItem));
+            put(s.d_events, plan.events.data(), plan.events.size() * sizeof(EventDesc));
+            put(s.d_hap_allele, plan.hap_allele.data(), plan.hap_allele.size());
+            if (plan.region_api) put(s.d_mapq, mapq, plan.n_reads);
+            put(s.d_rb, b.read_bases + plan.read_base0, plan.read_bases);
+            put(s.d_rq, b.read_qual + plan.read_base0, plan.read_bases);
+            if (!plan.region_api) {
+                put(s.d_ri, b.read_ins + plan.read_base0, plan.read_bases);
+                put(s.d_rd, b.read_del + plan.read_base0, plan.read_bases);
+                put(s.d_rc, b.read_gcp + plan.read_base0, plan.read_bases);
+            }
+            put(s.d_hb, b.hap_bases + plan.hap_base0, plan.hap_bases);
+            put_desc(s.pinned + sp.out_begin);
+            PHMM_CK(cudaMemcpyAsync(s.dev, s.pinned, sp.in_end, cudaMemcpyHostToDevice, s.main));
+            return PHMM_OK;
+        }
+    }
+    full_layout(s);
+    // stage descriptors + plan arrays in pinned memory, then copy
+    char* p = s.pinned;
+    size_t o = 0;
+    auto stage = [&](const void* src, size_t bytes) -> char* {
+        char* at = p + o;
+        if (bytes) std::memcpy(at, src, bytes);
+        o = align_up(o + std::max<size_t>(bytes, 1));
+        return at;
+    };
     char* desc = p;
-    std::memcpy(desc, &bd, sizeof(bd));
-    std::memcpy(desc + sizeof(bd), plan.classes.data(), sizeof(ClassDesc) * kNumClasses);
-    std::memset(desc + sizeof(bd) + sizeof(ClassDesc) * kNumClasses, 0, 4 * sizeof(unsigned int));
+    put_desc(desc);
     o = align_up(kDescBytes);
     char* h_regions = stage(plan.regions.data(), plan.regions.size() * sizeof(RegionDesc));
     char* h_read_off = stage(plan.read_off.data(), plan.read_off.size() * 8);
@@ -940,7 +1014,7 @@ phmm_status Engine::run(Slot& s, const Plan& plan, bool want_flags, bool restore
 phmm_status Engine::enqueue(Slot& s, const Plan& plan, const phmm_batch& b, bool want_flags, std::string& err,
                             const uint8_t* mapq, bool raw_sent)
 {
-    phmm_status st = upload(s, plan, b, err, mapq, raw_sent);
+    phmm_status st = upload(s, plan, b, err, mapq, raw_sent, /*may_compact=*/true);
     if (st != PHMM_OK) return st;
     return run(s, plan, want_flags, false, err);
 }
@@ -951,26 +1025,51 @@ phmm_status Engine::finish(Slot& s, const Plan& plan, double* out, uint8_t* pair
 {
     cudaStream_t m = s.main;
     char* desc = s.pinned;  // reuse the staged descriptor block for the read-back
-    PHMM_CK(cudaMemcpyAsync(desc, s.d_desc, kDescBytes, cudaMemcpyDeviceToHost, m));
-    if (plan.region_api) {
+    const bool compact = s.compact;
+    if (compact) {
+        // the descriptor block and every result behind it, to the second half of the staging
+        desc = s.pinned + kCompactBytes;
+        PHMM_CK(cudaMemcpyAsync(desc, s.dev + s.out_begin, s.out_bytes, cudaMemcpyDeviceToHost, m));
+    } else {
+        PHMM_CK(cudaMemcpyAsync(desc, s.d_desc, kDescBytes, cudaMemcpyDeviceToHost, m));
+    }
+    if (plan.region_api && !compact) {
         if (plan.n_reads && keep) PHMM_CK(cudaMemcpyAsync(keep, s.d_keep, plan.n_reads, cudaMemcpyDeviceToHost, m));
         if (plan.n_regions && n_kept)
             PHMM_CK(cudaMemcpyAsync(n_kept, s.d_nkept, plan.n_regions * sizeof(uint32_t), cudaMemcpyDeviceToHost, m));
     }
     if (!plan.events.empty()) {
-        if (gl) PHMM_CK(cudaMemcpyAsync(gl, s.d_gl, plan.gl_total * sizeof(double), cudaMemcpyDeviceToHost, m));
-        if (best) PHMM_CK(cudaMemcpyAsync(best, s.d_best, plan.events.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, m));
+        if (gl && !compact)
+            PHMM_CK(cudaMemcpyAsync(gl, s.d_gl, plan.gl_total * sizeof(double), cudaMemcpyDeviceToHost, m));
+        if (best && !compact) PHMM_CK(cudaMemcpyAsync(best, s.d_best, plan.events.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, m));
         if (allele_lk)
             PHMM_CK(cudaMemcpyAsync(allele_lk, s.d_allele_lk, plan.allele_lk_total * sizeof(double),
                                     cudaMemcpyDeviceToHost, m));
     }
-    if (plan.out_total && out) {
+    if (plan.out_total && out && !compact) {
         PHMM_CK(cudaMemcpyAsync(out, plan.region_api ? s.d_out2 : s.d_out, plan.out_total * sizeof(double),
                                 cudaMemcpyDeviceToHost, m));
         if (pair_flags) PHMM_CK(cudaMemcpyAsync(pair_flags, s.d_pair_flags, plan.out_total, cudaMemcpyDeviceToHost, m));
     }
     PHMM_CK(cudaEventRecord(s.ev_t3, m));
     PHMM_CK(cudaEventSynchronize(s.ev_t3));
+    if (compact) {
+        auto get = [&](void* dst, const void* src, size_t bytes) {
+            if (dst && bytes) std::memcpy(dst, desc + ((const char*)src - (s.dev + s.out_begin)), bytes);
+        };
+        if (plan.region_api) {
+            get(keep, s.d_keep, plan.n_reads);
+            get(n_kept, s.d_nkept, plan.n_regions * sizeof(uint32_t));
+        }
+        if (!plan.events.empty()) {
+            get(gl, s.d_gl, plan.gl_total * sizeof(double));
+            get(best, s.d_best, plan.events.size() * sizeof(int32_t));
+        }
+        if (out) {
+            get(out, plan.region_api ? s.d_out2 : s.d_out, plan.out_total * sizeof(double));
+            get(pair_flags, s.d_pair_flags, plan.out_total);
+        }
+    }
     const ClassDesc* cls = (const ClassDesc*)(desc + sizeof(BatchDesc));
     const unsigned int status = *(const unsigned int*)(desc + sizeof(BatchDesc) + sizeof(ClassDesc) * kNumClasses);
     uint64_t f64 = 0;

@@ -41,6 +41,8 @@ struct Slot {
     size_t pinned_bytes = 0;
     Capacity cap;
     Capacity floor;                  // the arena is never sized below this (serving slots pre-size)
+    bool compact = false;            // the arena holds a small batch in the compact layout
+    size_t out_begin = 0, out_bytes = 0;  // its results (descriptor block first) in the arena
     bool overlap = false;            // serving slot: over-subscribed FP32 grids, prioritised streams
     // carved device pointers
     BatchDesc* d_desc = nullptr;
@@ -113,8 +115,9 @@ public:
                        int32_t* best = nullptr, double* allele_lk = nullptr);
     // Upload only (descriptor, plan arrays, reads, haplotypes); then run the device pipeline, with
     // restore = true resetting the descriptor from its pristine device copy first (replays).
+    // may_compact: a small batch may be laid out compactly (one copy up, one back; not for replays).
     phmm_status upload(Slot& s, const Plan& plan, const phmm_batch& b, std::string& err,
-                       const uint8_t* mapq = nullptr, bool raw_sent = false);
+                       const uint8_t* mapq = nullptr, bool raw_sent = false, bool may_compact = false);
     // Copies a validated batch's bases and qualities into the slot's arena when it already holds
     // them (returns false, copying nothing, otherwise): the copies then overlap the host planning.
     bool upload_raw(Slot& s, const BatchScan& sc, const phmm_batch& b);
@@ -167,6 +170,7 @@ public:
 
 private:
     Engine() = default;
+    void full_layout(Slot& s);  // the arena's fixed sections, after a compact batch
     bool use_graph(const Plan& plan) const;  // replay the captured graph for this batch
     phmm_status ensure_capacity(Slot& s, const Plan& plan, std::string& err);
     phmm_status launch_pipeline(Slot& s, bool want_flags, const Plan* plan, const TileTable& tiles, std::string& err);

@@ -15,14 +15,18 @@
 namespace phmm {
 
 // ------------------------------------------------------------------------------------------
-// Haplotype bytes -> per-variant match codes (grid-stride).
+// Before the passes (grid-stride): haplotype bytes -> per-variant match codes, and the output reset:
+// every likelihood NaN (pairs with an empty read or haplotype stay NaN), flags 0.  One launch for both: a
+// small batch waits for each (about 3 us), and a large one streams both through HBM either way.
 // ------------------------------------------------------------------------------------------
-__global__ void prep_codes_kernel(const BatchDesc* __restrict__ desc, const uint8_t* __restrict__ hap_bases,
-                                  uint32_t* __restrict__ codes_inter, uint32_t* __restrict__ codes_intra)
+__global__ void prep_kernel(const BatchDesc* __restrict__ desc, const uint8_t* __restrict__ hap_bases,
+                            uint32_t* __restrict__ codes_inter, uint32_t* __restrict__ codes_intra,
+                            double* __restrict__ out, uint8_t* __restrict__ flags)
 {
     const uint64_t total = desc->hap_bases_total;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint64_t i = first; i < total; i += stride) {
         const uint8_t b = hap_bases[i];
         codes_inter[kCodePad + i] = hap_code(b, kInter);
         codes_intra[kCodePad + i] = hap_code(b, kIntra);
@@ -36,18 +40,9 @@ __global__ void prep_codes_kernel(const BatchDesc* __restrict__ desc, const uint
             codes_intra[kCodePad + total + k] = 0u;
         }
     }
-}
-
-// ------------------------------------------------------------------------------------------
-// Output reset: every likelihood NaN (pairs with an empty read or haplotype stay NaN), flags 0.
-// ------------------------------------------------------------------------------------------
-__global__ void reset_outputs_kernel(const BatchDesc* __restrict__ desc, double* __restrict__ out,
-                                     uint8_t* __restrict__ flags)
-{
-    const uint64_t total = desc->out_total;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t outs = desc->out_total;
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    for (uint64_t i = first; i < outs; i += stride) {
         out[i] = nan;
         if (flags) flags[i] = 0;
     }
@@ -156,9 +151,7 @@ static const F64Kernel kF64Check[2 * 9] = {PHMM_ROW64_CHECK(kInter), PHMM_ROW64_
 cudaError_t launch_prep(const BatchDesc* desc, const uint8_t* hap_bases, uint32_t* codes_inter, uint32_t* codes_intra,
                         double* out, uint8_t* flags, int num_sms, cudaStream_t st)
 {
-    const int threads = 256;
-    reset_outputs_kernel<<<num_sms * 4, threads, 0, st>>>(desc, out, flags);
-    prep_codes_kernel<<<num_sms * 4, threads, 0, st>>>(desc, hap_bases, codes_inter, codes_intra);
+    prep_kernel<<<num_sms * 8, 256, 0, st>>>(desc, hap_bases, codes_inter, codes_intra, out, flags);
     return cudaGetLastError();
 }
 
