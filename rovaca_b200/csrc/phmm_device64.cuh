@@ -13,8 +13,6 @@
 // instead of 4 K + 3, two shuffles instead of three, and (PM_EQ) 7 operations per cell instead of 8.
 #pragma once
 
-#include <type_traits>
-
 #include "phmm_device.cuh"
 
 namespace phmm {
@@ -29,27 +27,7 @@ struct LaneRowsEq {
     double xxn;                     // xx of the row below the lane (1 for a pad row)
     double mm, gm, mx;              // one value per read (mx == my)
     uint32_t padmask;               // bit k: slot k is a pad row
-    int shrink;                     // step_shrink of the lane's rows
 };
-
-__device__ __forceinline__ int larger(int a, int b) { return a > b ? a : b; }
-
-// v >= 2^-bits_below(v) for a probability v > 0; 0 for v = 0 (its products are exactly 0).
-__device__ __forceinline__ int bits_below(double v)
-{
-    return v > 0.0 ? 1023 - (int)((uint32_t)__double2hiint(v) >> 20) : 0;
-}
-
-// The bits by which one step can shrink a value at most: every nonzero result of a step, intermediate
-// ones included, is at least the smallest nonzero input times 2^-shrink.  Its longest product is M of the
-// lane's first row (prior, at least 2^-prior), carried by M * mx into the insertion chain (gap), down the
-// lane's K rows and to the row below (K factors xx, at least 2^-cont each), and into a diagonal sum (a
-// factor mm or gapm, at least 2^-keep); the last bit covers the roundings (under K + 4 of 2^-53 each).
-template <int K>
-__device__ __forceinline__ int step_shrink(int prior, int gap, int cont, int keep)
-{
-    return prior + gap + K * cont + keep + 1;
-}
 
 // Loads this lane's rows of the stripe starting at padded row first_padded_row (pad rows above the
 // read) and writes their priors to the warp's table.  Returns true when one of the lane's rows is an
@@ -73,7 +51,6 @@ __device__ __forceinline__ bool load_rows_eq(LaneRowsEq<K>& L, double* tab, cons
     const int below = first_padded_row + lane * K + K - pad;
     L.xxn = below >= 0 && below < R ? tb.ph2pr[b.read_c[roff + (uint64_t)below] & 127] : 1.0;
     L.In = L.Sn = L.Mb = L.Ib = 0.0;
-    int prior_bits = 0, cont_bits = bits_below(L.xxn);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         L.S[k] = L.Dn[k] = 0.0;
@@ -86,8 +63,6 @@ __device__ __forceinline__ bool load_rows_eq(LaneRowsEq<K>& L, double* tab, cons
             pa = tb.pmat[q];
             pb = (V == kInter) ? tb.pmis_inter[q] : tb.pmis_intra[q];
             L.xx[k] = tb.ph2pr[b.read_c[o] & 127];
-            prior_bits = larger(prior_bits, larger(bits_below(pa), bits_below(pb)));
-            cont_bits = larger(cont_bits, bits_below(L.xx[k]));
             const uint8_t base = b.read_bases[o];
             rc = match_code(base, V);
             if (V == kInter) exotic |= base_class(base) == 4u;
@@ -99,7 +74,6 @@ __device__ __forceinline__ bool load_rows_eq(LaneRowsEq<K>& L, double* tab, cons
         for (int c = 0; c < kTabClasses; ++c)
             tab[prior_slot<K>((uint32_t)c, k, lane)] = class_matches((uint32_t)c, rc, V) ? pa : pb;
     }
-    L.shrink = step_shrink<K>(prior_bits, bits_below(L.mx), cont_bits, larger(bits_below(L.mm), bits_below(L.gm)));
     return exotic;
 }
 
@@ -115,7 +89,6 @@ struct LaneRowsRow {
     double xx[K], mm[K], gm[K], mx[K], my[K];
     double xxn, mmn, gmn, mxn;      // the row below the lane (xx 1 and the rest 0 for a pad row)
     uint32_t padmask;
-    int shrink;
 };
 
 template <int K, int V>
@@ -143,8 +116,6 @@ __device__ __forceinline__ bool load_rows_row(LaneRowsRow<K>& L, double* tab, co
     };
     double myn;
     params(first_padded_row + lane * K + K - pad, L.xxn, L.mmn, L.gmn, L.mxn, myn);
-    int prior_bits = 0, cont_bits = bits_below(L.xxn), gap_bits = bits_below(L.mxn);
-    int keep_bits = larger(bits_below(L.mmn), bits_below(L.gmn));
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         L.S[k] = L.Dn[k] = 0.0;
@@ -160,18 +131,13 @@ __device__ __forceinline__ bool load_rows_row(LaneRowsRow<K>& L, double* tab, co
             const uint8_t base = b.read_bases[o];
             rc = match_code(base, V);
             if (V == kInter) exotic |= base_class(base) == 4u;
-            prior_bits = larger(prior_bits, larger(bits_below(pa), bits_below(pb)));
         } else {
             L.padmask |= 1u << k;
         }
-        cont_bits = larger(cont_bits, bits_below(L.xx[k]));
-        gap_bits = larger(gap_bits, larger(bits_below(L.mx[k]), bits_below(L.my[k])));
-        keep_bits = larger(keep_bits, larger(bits_below(L.mm[k]), bits_below(L.gm[k])));
 #pragma unroll
         for (int c = 0; c < kTabClasses; ++c)
             tab[prior_slot<K>((uint32_t)c, k, lane)] = class_matches((uint32_t)c, rc, V) ? pa : pb;
     }
-    L.shrink = step_shrink<K>(prior_bits, gap_bits, cont_bits, keep_bits);
     return exotic;
 }
 
@@ -254,36 +220,25 @@ __device__ __forceinline__ double row_diag(const LaneRowsRow<K>& L, int k, doubl
     return diag_eq<V, true>(L.gm[k], L.mm[k], dgM, dgI, dgD);
 }
 
-// The smallest nonzero value among the inputs of the lane's next step, by its high word less 1 (a zero
-// wraps to the largest): its rows' pending sums and next-column D, and the two values it hands the lane
-// below (that lane's first-row inputs).  Flushed values are 0 or normal, so a zero high word means 0.
-// Taken as a tree (depth log2(2 K + 2) instead of a chain of 2 K + 2 dependent operations).
-template <int K, typename LR>
-__device__ __forceinline__ uint32_t rows_min_hi(const LR& L)
-{
-    constexpr int N = 2 * K + 2;
-    uint32_t v[N];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        v[2 * k] = (uint32_t)__double2hiint(L.S[k]) - 1u;
-        v[2 * k + 1] = (uint32_t)__double2hiint(L.Dn[k]) - 1u;
-    }
-    v[2 * K] = (uint32_t)__double2hiint(L.In) - 1u;
-    v[2 * K + 1] = (uint32_t)__double2hiint(L.Sn) - 1u;
-#pragma unroll
-    for (int w = 1; w < N; w *= 2) {
-#pragma unroll
-        for (int i = 0; i + w < N; i += 2 * w) v[i] = min(v[i], v[i + w]);
-    }
-    return v[0];
-}
+// The pass sweeps without flushes first.  A result below 2^-1022 that the reference flushes to 0 is then
+// kept, which can only matter to values near it: every operation adds products with factors of at most 1,
+// so what the flushes take away stays below about 2^-1000 in any later value, and a value of 2^-700 or
+// more, which has no bits below 2^-753, is the same with and without it (but for a sum that falls exactly
+// on a rounding tie).  A pair whose sum is below 2^-700, a likelihood below 1e-517, is swept again with the
+// reference's flush after every operation; so is one whose sum is 0.
+// Before, every step either flushed (about three integer operations per FP64 operation, more than the
+// FP64 work itself) or ran without under a warp vote that no result could fall below 2^-1022, which long
+// reads rarely pass: far from a read's alignment there are always values around 2^-1022.  Measured on
+// B200, FP64 pass of 24 regions of reads of 257-768 bases 6.2 ms then, 3.0 ms now; of 60 low-quality regions
+// 25.1 and 22.6 ms.
+constexpr double kUnflushedMin = 0x1p-700;
 
 // Sweep one stripe over the column stream of haplotypes [g_lo, g_hi): as `sweep` (phmm_device.cuh),
 // the scratch row holding the handed-on (I, sum) pair per column.  LR: LaneRowsEq or LaneRowsRow.
-template <int K, int V, bool FROM_SCR, bool TO_SCR, typename LR>
+template <int K, int V, bool FROM_SCR, bool TO_SCR, bool FLUSH, typename LR>
 __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTables<double>& tb,
                          const SweepOut& so, uint32_t g_lo, uint32_t g_hi, double* scr, int lane, bool above_row0,
-                         bool exotic, uint64_t roff, int R, int row0)
+                         bool exotic, uint64_t roff, int R, int row0, uint32_t& again_lo, uint32_t& again_hi)
 {
     const uint64_t s0 = b.hap_off[g_lo];
     const int Tcols = (int)(b.hap_off[g_hi] - s0);
@@ -296,29 +251,13 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
     double D0 = 0.0;
     double Stop = 0.0;  // lane 0's first-row sum below the boundary row (M = I = 0, D = C/H)
     double sumM = 0.0, sumI = 0.0;
-    // Steps run in chunks of four, with the flushes of every result or, when the vote has shown that no
-    // result of the chunk can fall below 2^-1022, without.  The vote is taken in the middle of the chunk
-    // before, so that the steps behind it cover its latency (the chunk's branch waits on it), on the bound
-    // of the six steps up to the chunk's end.  The bound follows from the item's own probabilities
-    // (step_shrink): about 65 bits a step for 8 rows a lane and qualities up to 45, where the smallest
-    // probability of any quality would give 396.  Measured on B200, FP64 pass of 60 low-quality regions:
-    // 26.1 ms with a vote per two steps on that smallest-probability bound, 25.1 ms so.
-    bool flush_free = false, free_next = false;
     uint32_t wn = codes[-lane];  // the code word of the lane's next column, loaded a step ahead
-
-    int shrink = L.shrink;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) shrink = larger(shrink, __shfl_sync(0xffffffffu, shrink, lane ^ o));
-    constexpr int kAhead = kChunkScalar / 2 + kChunkScalar;  // steps a vote covers
-    const uint32_t free_hi = 1 + kAhead * shrink < 2046 ? ((uint32_t)(1 + kAhead * shrink) << 20) - 1u : 0xffffffffu;
 
     const int steps = Tcols + kWarp;
     // Stripes after the first: the row above (scratch, one 16-byte pair per column) comes through a ring
-    // in shared memory, copied two blocks ahead, so that lane 0 does not wait for L2 in every step and
-    // the vote can look at the values the next steps will take (FP64 pass of 24 regions of long reads 6.6
-    // and 6.2 ms; far from a read's alignment there are always values near 2^-1022, so most steps of long
-    // reads keep their flushes).  Lane 31 writes the same row 31 columns
-    // behind lane 0 (for the stripe below), never a column still to be read.
+    // in shared memory, copied two blocks ahead, so that lane 0 does not wait for L2 in every step.
+    // Lane 31 writes the same row 31 columns behind lane 0 (for the stripe below), never a column still
+    // to be read.
     static_assert(!FROM_SCR || K == kMaxK, "the ring is part of the multi-stripe shape's table");
     double* ring = tab + kTabClasses * K * kWarp;
     auto copy_block = [&](int c0) {
@@ -340,6 +279,10 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
                 const double tot = radd(sumM, sumI);
                 const uint64_t oi = so.out_base + (uint64_t)(cur - g_lo) * so.out_stride;
                 so.out[oi] = log10(tot) - Scale<double>::log10_initial();
+                if (!FLUSH && !(tot >= kUnflushedMin)) {  // to be swept again (lane 31's range)
+                    if (again_lo == again_hi) again_lo = cur;
+                    again_hi = cur + 1;
+                }
             }
             ++cur;
         }
@@ -368,9 +311,7 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
         }
     };
 
-    constexpr bool kVote = PHMM_F64_VOTE;
-    auto step = [&](int t, bool check, auto flush) {
-        constexpr bool FL = decltype(flush)::value;
+    auto step = [&](int t, bool check) {
         const int p = t - lane;
         double uI = shfl_up1(L.In);
         double uS = shfl_up1(L.Sn);
@@ -400,7 +341,7 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
                 if (i >= 0 && i < R && b.read_bases[roff + i] == hb) pr[k] = tb.pmat[b.read_q[roff + i] & 127];
             }
         }
-        cells_eq<K, V, FL>(L, pr, uI, uS);
+        cells_eq<K, V, FLUSH>(L, pr, uI, uS);
         if (TO_SCR) {
             if (lane == kWarp - 1 && p >= 0 && p < Tcols) {
                 scr[2 * p + 0] = L.In;
@@ -410,23 +351,8 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
             sumM = radd(sumM, L.Mb);
             sumI = radd(sumI, L.Ib);
         }
-        if constexpr (kVote) {
-            if (t % kChunkScalar == kChunkScalar / 2 - 1) {
-                uint32_t v = rows_min_hi<K>(L);
-                if (FROM_SCR && lane < kAhead && t + 1 + lane < Tcols) {  // lane 0's inputs of the covered steps
-                    const double* q = ring + 2 * ((t + 1 + lane) & (kScrRing64 - 1));
-                    v = min(v, min((uint32_t)__double2hiint(q[0]) - 1u, (uint32_t)__double2hiint(q[1]) - 1u));
-                }
-                free_next = __all_sync(0xffffffffu, v >= free_hi);
-            } else if (t % kChunkScalar == kChunkScalar - 1) {
-                flush_free = free_next;
-            }
-        }
     };
-    static_assert(kChunkScalar % 2 == 0 && kScrBlock64 % kChunkScalar == 0 && kAhead <= kScrBlock64 && kAhead <= kWarp,
-                  "a vote looks at most one block ahead");
-    const auto yes = std::true_type{};
-    const auto no = std::false_type{};
+    static_assert(kScrBlock64 % kChunkScalar == 0, "a block of the ring is whole chunks");
 
     for (int t0 = 0; t0 < steps; t0 += kChunkScalar) {
         if (FROM_SCR && t0 % kScrBlock64 == 0) {  // columns up to t0 + 2 blocks are complete from here
@@ -436,19 +362,11 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
         }
         const int nb31 = __shfl_sync(0xffffffffu, nb, kWarp - 1);
         if (nb31 >= t0 + kChunkScalar && t0 + kChunkScalar <= steps) {
-            if (kVote && flush_free) {
 #pragma unroll
-                for (int u = 0; u < kChunkScalar; ++u) step(t0 + u, false, no);
-            } else {
-#pragma unroll
-                for (int u = 0; u < kChunkScalar; ++u) step(t0 + u, false, yes);
-            }
+            for (int u = 0; u < kChunkScalar; ++u) step(t0 + u, false);
         } else {
             for (int u = 0; u < kChunkScalar; ++u)
-                if (t0 + u < steps) {
-                    if (kVote && flush_free) step(t0 + u, true, no);
-                    else step(t0 + u, true, yes);
-                }
+                if (t0 + u < steps) step(t0 + u, true);
         }
     }
     if (FROM_SCR) {

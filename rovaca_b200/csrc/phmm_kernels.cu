@@ -53,13 +53,12 @@ __global__ void prep_kernel(const BatchDesc* __restrict__ desc, const uint8_t* _
 // claim, streamed through the read like an FP32 work item.
 // ------------------------------------------------------------------------------------------
 // Resident warps per SM of the FP64 classes of mode 0 (constant gaps, insertion = deletion), the
-// compiler's register bound: 8 rows per lane at 12 warps (168 registers, no spills), 7 rows at 16
-// (128 registers, 48 bytes of spill loads).  Measured on B200 with the two-value lane state: 8 rows
-// at 12 warps ran the underflow-stress shape's FP64 pass in 43.7 ms against 44.9 at 16, and the
-// benchmark batch's 8-row class in 8.8 against 9.1 ms; 7 rows ran 5.1 ms at 16 against 5.3 at 12.
-// The other classes keep what they need.  Build-time settings.
+// compiler's register bound: 16 (128 registers; 296 and 64 bytes of spill loads for 8 and 7 rows per lane).
+// Measured on B200 with the unflushed sweep, 8 rows: the FP64 pass of 60 low-quality regions 22.6 ms at 16
+// warps, 23.0 at 12, 23.6 at 11; of the 1,000-region batch 4.54 and 4.63 ms at 16 and 12; 7 rows 2.80 ms
+// at 16 and 2.87 at 12.  The other classes keep what they need.  Build-time settings.
 #ifndef PHMM_F64_MIN_WARPS_K8
-#define PHMM_F64_MIN_WARPS_K8 12
+#define PHMM_F64_MIN_WARPS_K8 16
 #endif
 #ifndef PHMM_F64_MIN_WARPS_K7
 #define PHMM_F64_MIN_WARPS_K7 16

@@ -12,6 +12,47 @@
 namespace phmm {
 
 // ------------------------------------------------------------------------------------------
+// One read against a run of haplotypes [g_lo, g_hi) in the recompute pass: the two-value lane state
+// (phmm_device64.cuh), one value per read for constant gaps with insertion = deletion, per row otherwise.
+// FLUSH: with the flush after every operation; without it, [again_lo, again_hi) of lane 31 receives the
+// haplotypes to be run again with it.
+// ------------------------------------------------------------------------------------------
+template <int K, int V, int PM, bool MULTI, bool FLUSH>
+__device__ __forceinline__ void run_stripes(const BatchView& b, const ProbTables<double>& tb, const SweepOut& so,
+                                            uint32_t g_lo, uint32_t g_hi, int lane, double* scr, double* tab,
+                                            uint64_t roff, int R, uint32_t& again_lo, uint32_t& again_hi)
+{
+    using LR = typename std::conditional<PM == PM_EQ, LaneRowsEq<K>, LaneRowsRow<K>>::type;
+    LR L;
+    constexpr int SR = kWarp * K;  // rows per stripe
+    const int stripes = MULTI ? (R + SR - 1) / SR : 1;
+    const int pad = SR * stripes - R;
+    for (int s = 0; s < stripes; ++s) {
+        bool exotic;
+        if constexpr (PM == PM_EQ)
+            exotic = load_rows_eq<K, V>(L, tab, b, tb, roff, R, s * SR, pad, lane);
+        else
+            exotic = load_rows_row<K, V>(L, tab, b, tb, roff, R, s * SR, pad, lane);
+        const bool above_row0 = (s == 0) && (lane * K <= pad);
+        const int row0 = s * SR - pad;  // read position of slot 0 of lane 0
+        if constexpr (!MULTI)
+            sweep_eq<K, V, false, false, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R,
+                                                row0, again_lo, again_hi);
+        else if (s == 0)
+            sweep_eq<K, V, false, true, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R,
+                                               row0, again_lo, again_hi);
+        else if (s == stripes - 1)
+            sweep_eq<K, V, true, false, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R,
+                                               row0, again_lo, again_hi);
+        else
+            sweep_eq<K, V, true, true, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R,
+                                              row0, again_lo, again_hi);
+        // lane 31's scratch row is read by lane 0 in the next stripe; every lane's priors are rewritten
+        __syncwarp();
+    }
+}
+
+// ------------------------------------------------------------------------------------------
 // One read against a run of haplotypes [g_lo, g_hi).
 // ------------------------------------------------------------------------------------------
 template <typename T, int K, int V, int PM, bool MULTI, bool UNF = false>
@@ -28,31 +69,15 @@ __device__ __forceinline__ void run_read(const BatchView& b, const ProbTables<T>
         return;
     }
     if constexpr (PM == PM_EQ || (PM == PM_ROW && !UNF)) {
-        // the recompute pass: the two-value lane state (phmm_device64.cuh), one value per read for
-        // constant gaps with insertion = deletion, per row otherwise
         static_assert(sizeof(T) == 8 && !UNF, "the two-value lane state is the FP64 recompute");
-        using LR = typename std::conditional<PM == PM_EQ, LaneRowsEq<K>, LaneRowsRow<K>>::type;
-        LR L;
-        constexpr int SR = kWarp * K;  // rows per stripe
-        const int stripes = MULTI ? (R + SR - 1) / SR : 1;
-        const int pad = SR * stripes - R;
-        for (int s = 0; s < stripes; ++s) {
-            bool exotic;
-            if constexpr (PM == PM_EQ)
-                exotic = load_rows_eq<K, V>(L, tab, b, tb, roff, R, s * SR, pad, lane);
-            else
-                exotic = load_rows_row<K, V>(L, tab, b, tb, roff, R, s * SR, pad, lane);
-            const bool above_row0 = (s == 0) && (lane * K <= pad);
-            const int row0 = s * SR - pad;  // read position of slot 0 of lane 0
-            if constexpr (!MULTI)
-                sweep_eq<K, V, false, false>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R, row0);
-            else if (s == 0)
-                sweep_eq<K, V, false, true>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R, row0);
-            else if (s == stripes - 1)
-                sweep_eq<K, V, true, false>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R, row0);
-            else
-                sweep_eq<K, V, true, true>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R, row0);
-            if (MULTI) __syncwarp();  // lane 31's scratch row is read by lane 0 in the next stripe
+        uint32_t again_lo = 0, again_hi = 0;
+        run_stripes<K, V, PM, MULTI, false>(b, tb, so, g_lo, g_hi, lane, scr, tab, roff, R, again_lo, again_hi);
+        again_lo = __shfl_sync(0xffffffffu, again_lo, kWarp - 1);
+        again_hi = __shfl_sync(0xffffffffu, again_hi, kWarp - 1);
+        if (again_lo != again_hi) {
+            SweepOut so2 = so;
+            so2.out_base += (uint64_t)(again_lo - g_lo) * so.out_stride;
+            run_stripes<K, V, PM, MULTI, true>(b, tb, so2, again_lo, again_hi, lane, scr, tab, roff, R, again_lo, again_hi);
         }
     } else {
         LaneRows<T, K, PM> L;

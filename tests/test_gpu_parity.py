@@ -195,6 +195,38 @@ def test_random_lengths_all_classes(engine, oracle):
     assert np.array_equal(flags.astype(bool), used)
 
 
+@pytest.mark.parametrize("length", [120, 250, 256, 400, 520])
+@pytest.mark.parametrize("gaps", ["constant", "per_base"])
+def test_tiny_likelihoods_equal_the_oracle(engine, oracle, length, gaps):
+    """Reads unrelated to their haplotypes, at qualities that take the likelihoods from those FP32 holds
+    over 1e-517, where the FP64 pass turns to flushing every operation, to values below all doubles: the
+    oracle's bits and decisions."""
+    rng = np.random.default_rng(length)
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    haps = [acgt[rng.integers(0, 4, 60 + 30 * h)].tobytes() for h in range(6)]
+    reads, q, i, d, c = [], [], [], [], []
+    for r in range(24):
+        own = np.frombuffer(haps[r % 6][:length], np.uint8)
+        x = acgt[rng.integers(0, 4, length)].copy()
+        n = int(len(own) * (r % 4) / 4)      # a share of the read that does match
+        x[:n] = own[:n]
+        reads.append(x.tobytes())
+        hi = 4 + 2 * r
+        q.append(rng.integers(2, hi, length).astype(np.uint8).tobytes())
+        vary = gaps == "per_base"
+        i.append((rng.integers(20, 60, length) if vary else np.full(length, 10 + 2 * r)).astype(np.uint8).tobytes())
+        d.append((rng.integers(20, 60, length) if vary else np.full(length, 10 + 2 * r)).astype(np.uint8).tobytes())
+        c.append((rng.integers(8, 30, length) if vary else np.full(length, 10 + r)).astype(np.uint8).tobytes())
+    pb = PackedBatch.from_regions([Region(haps, reads, q, i, d, c)])
+    got, flags, _ = engine.compute(pb, want_flags=True)
+    want, used = oracle.batch(pb)
+    assert_same_values(got, want, EXACT)
+    assert np.array_equal(flags.astype(bool), used)
+    if length == 400:
+        finite = want[np.isfinite(want)]
+        assert finite.min() < -530 and finite.max() > -450
+
+
 def test_chunked_compute_equals_one_pipeline(oracle):
     """phmm_compute_regions run as a pipeline of region chunks on two device slots (chunk_cells
     forced down) gives the likelihoods, flags and counts of one pipeline, again when a second call
