@@ -13,10 +13,11 @@
 //
 // Arithmetic.  Scores are stored with a bias that makes every half non-negative, so that a packed add
 // or subtract is one plain 32-bit instruction (no borrow crosses the halves) and only the maxima are
-// packed instructions.  The four choices of a cell (E opened or extended, F likewise, insertion taken,
-// deletion taken) come out as sign bits of 0x8000 + a - max(a, b); a byte permute that replicates the
-// signs collects two of them for both alignments, one AND-OR deposits them: 4 operations per packed
-// cell for the codes, 16 in all, 8 per cell against about 21 in the 32-bit kernel.
+// packed instructions.  The four facts of a cell (E extended, F extended, H equals the diagonal term, H
+// equals E; a tie goes to the diagonal, then to the insertion, as the reference's strict comparisons have
+// it) come out as sign bits of 0x8000 + a - max; a byte permute that replicates the signs collects two of
+// them for both alignments, one AND-OR deposits them: 4 operations per packed cell for the codes, 15 in
+// all, 7.5 per cell against about 21 in the 32-bit kernel.
 // The substitution scores come from a per-lane table in shared memory (6 base classes x K columns per
 // alignment: A, C, G, T, N, any other byte) read at the row's class, one permute per packed cell to
 // join the halves; a read with a byte outside A/C/G/T/N runs the comparing form of the step.
@@ -36,12 +37,7 @@
 namespace phmm {
 
 #ifdef __CUDA_ARCH__
-__device__ __forceinline__ uint32_t sw_max2(uint32_t a, uint32_t b)
-{
-    uint32_t d;
-    asm("max.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
+__device__ __forceinline__ uint32_t sw_max3(uint32_t a, uint32_t b, uint32_t c) { return __vimax3_u16x2(a, b, c); }
 // max(a + b, c) per half (the add wraps per half: b may be a negated constant)
 __device__ __forceinline__ uint32_t sw_addmax2(uint32_t a, uint32_t b, uint32_t c) { return __viaddmax_u16x2(a, b, c); }
 template <uint32_t SEL>
@@ -58,6 +54,7 @@ __device__ inline uint32_t sw_max2(uint32_t a, uint32_t b)
     const uint32_t h = (a >> 16) > (b >> 16) ? a >> 16 : b >> 16;
     return l | (h << 16);
 }
+__device__ inline uint32_t sw_max3(uint32_t a, uint32_t b, uint32_t c) { return sw_max2(sw_max2(a, b), c); }
 __device__ inline uint32_t sw_addmax2(uint32_t a, uint32_t b, uint32_t c)
 {
     return sw_max2(((a + b) & 0xffffu) | ((a & 0xffff0000u) + (b & 0xffff0000u)), c);
@@ -348,10 +345,9 @@ __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int 
                 const uint32_t fe = Fp[k] - XE;
                 const uint32_t f = sw_addmax2(Hp[k], NO, fe);
                 const uint32_t hr = diag + sc + MM;
-                const uint32_t h1 = sw_max2(hr, e);
-                const uint32_t h2 = sw_max2(h1, f);
+                const uint32_t h2 = sw_max3(hr, e, f);
                 const uint32_t w1 = sw_prmt<0xFDB9>(kSign + ee - e, kSign + fe - f);    // extended: E, F
-                const uint32_t w2 = sw_prmt<0xFDB9>(kSign + hr - h1, kSign + h1 - h2);  // not taken: I, D
+                const uint32_t w2 = sw_prmt<0xFDB9>(kSign + hr - h2, kSign + e - h2);   // H is the diagonal, is E
                 code[k / 4] |= w1 & (0x01010101u << (2 * (k & 3)));
                 code[k / 4] |= w2 & (0x02020202u << (2 * (k & 3)));
                 diag = Hp[k];
@@ -456,13 +452,13 @@ __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int 
     while (__any_sync(0xffffffffu, i > 0 && j > 0)) {
         const int ci = i - (state == 1 ? 0 : l16), cj = j - (state == 2 ? 0 : l16);
         const bool in = ci > 0 && cj > 0 && i > 0 && j > 0;
-        uint32_t b = 0;  // bit 0 E extended, 1 insertion not taken, 2 F extended, 3 deletion not taken
+        uint32_t b = 0;  // bit 0 E extended, 1 H is the diagonal term, 2 F extended, 3 H is E
         if (in) {
             const int s = cj - 1 + pad, ln = s / K, k = s - ln * K;
             const uint32_t w = bt[(uint32_t)(ci - 1 + ln) * ROW + (k >> 2) * 32 + ln] >> (8 * q + 2 * (k & 3));
             b = (w & 3u) | ((w >> 14) & 12u);
         }
-        const bool go = in && (state == 0 ? (b & 10u) == 10u : state == 1 ? (b & 1u) != 0 : (b & 4u) != 0);
+        const bool go = in && (state == 0 ? (b & 2u) != 0 : state == 1 ? (b & 1u) != 0 : (b & 4u) != 0);
         const uint32_t valid = (__ballot_sync(0xffffffffu, in) >> base) & 0xffffu;
         const uint32_t run = (__ballot_sync(0xffffffffu, go) >> base) & 0xffffu;
         const uint32_t b0 = __shfl_sync(0xffffffffu, b, base);
@@ -474,7 +470,7 @@ __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int 
                     push(0, n);
                     i -= n;
                     j -= n;
-                } else if ((b0 & 8u) == 0) {
+                } else if ((b0 & 8u) == 0) {  // above the diagonal term and E: a deletion
                     push(2, 1);
                     --i;
                     state = b0 & 4u ? 2 : 0;
