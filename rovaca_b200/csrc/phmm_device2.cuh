@@ -383,16 +383,22 @@ struct SweepOut2 {
 };
 
 // Sweep one stripe of both reads over the column stream of haplotypes [g_lo, g_hi).
-//   FROM_SCR: the row above lane 0 comes from the warp's scratch row (stripe > 0).
-//   TO_SCR:   lane 31's bottom rows go to the scratch row (not the last stripe).
+//   from_scr: the row above lane 0 comes from the warp's scratch row (stripe > 0).
+//   to_scr:   lane 31's bottom rows go to the scratch row (not the last stripe).
+// MULTI: the stripe is one of several, and both are read at run time; single-stripe kernels have neither.
+// (One sweep for all stripes: the warps of an SM are at different stripes, and a sweep of its own for
+// first, middle and last ones was three times the code.  Measured on B200, FP32 pass of 24 regions of long
+// reads: 6.9 ms with three, 6.5 ms with one.)
 // first: the stripe's first padded row.  aboveX / aboveY: the row above the lane's first row is
 // row 0 or a pad row, per read.  exotic: the warp holds an inter row with a byte outside A/C/G/T
 // (every step runs the checked path).
-template <int KH, int V, int PM, bool FROM_SCR, bool TO_SCR>
+template <int KH, int V, int PM, bool MULTI>
 __device__ void sweep2(LaneRows2<KH, PM>& L, float4* tab, const BatchView& b, const ProbTables<float>& tb,
                        const PassControl& pc, const SweepOut2& so, const ReadPair& rp, int first, uint32_t g_lo,
-                       uint32_t g_hi, float2* scr, int lane, bool aboveX, bool aboveY, bool exotic)
+                       uint32_t g_hi, float2* scr, int lane, bool aboveX, bool aboveY, bool exotic, bool from_scr,
+                       bool to_scr)
 {
+    const bool FROM_SCR = MULTI && from_scr, TO_SCR = MULTI && to_scr;
     constexpr int QJ = tab_quads<KH>();
     const uint64_t s0 = b.hap_off[g_lo];
     const int Tcols = (int)(b.hap_off[g_hi] - s0);
@@ -401,7 +407,7 @@ __device__ void sweep2(LaneRows2<KH, PM>& L, float4* tab, const BatchView& b, co
     // the warp's code ring follows its prior table (PHMM_CODES_STAGED)
     uint32_t* ring = reinterpret_cast<uint32_t*>(tab + tab_floats4<KH>());
     // and the ring of the row above the stripe the code ring
-    constexpr bool ROW_RING = FROM_SCR && PM != PM_ALL;
+    const bool ROW_RING = FROM_SCR && PM != PM_ALL;
     float4* row_ring = tab + tab_floats4<KH>() + kCodeRingFloat4;
     const float C = Scale<float>::initial();
     const bool writer = lane == kWarp - 1;
@@ -542,21 +548,23 @@ __device__ void sweep2(LaneRows2<KH, PM>& L, float4* tab, const BatchView& b, co
         }
         if (check && p == nb) boundary();
         if (lane == 0) {
-            if (FROM_SCR) {
-                const bool ok = p >= 0 && p < Tcols;
-                if (ROW_RING) {
-                    const float4 q = row_ring[p & (kScrRing - 1)];
-                    uI = ok ? f2(q.x, q.y) : f2(0.f, 0.f);
-                    uD = ok ? f2(q.z, q.w) : f2(0.f, 0.f);
-                } else {
-                    uM = ok ? scr[3 * p + 0] : f2(0.f, 0.f);
-                    uI = ok ? scr[3 * p + 1] : f2(0.f, 0.f);
-                    uD = ok ? scr[3 * p + 2] : f2(0.f, 0.f);
-                }
-            } else if (HANDOFF) {
+            if (HANDOFF) {
                 // below the boundary row (M = I = 0, D = C/H): I = fma(0, xx, 0 * mx) = 0
                 uI = f2(0.f, 0.f);
                 uD = Stop;
+                if (MULTI) {
+                    const float4 q = row_ring[p & (kScrRing - 1)];
+                    if (FROM_SCR) {
+                        const bool ok = p >= 0 && p < Tcols;
+                        uI = ok ? f2(q.x, q.y) : f2(0.f, 0.f);
+                        uD = ok ? f2(q.z, q.w) : f2(0.f, 0.f);
+                    }
+                }
+            } else if (FROM_SCR) {
+                const bool ok = p >= 0 && p < Tcols;
+                uM = ok ? scr[3 * p + 0] : f2(0.f, 0.f);
+                uI = ok ? scr[3 * p + 1] : f2(0.f, 0.f);
+                uD = ok ? scr[3 * p + 2] : f2(0.f, 0.f);
             } else {
                 uM = f2(0.f, 0.f);
                 uI = f2(0.f, 0.f);
@@ -602,10 +610,9 @@ __device__ void sweep2(LaneRows2<KH, PM>& L, float4* tab, const BatchView& b, co
                     scr[3 * p + 2] = L.Db;
                 }
             }
-        } else {
-            sumM = radd2(sumM, L.Mb);
-            sumI = radd2(sumI, L.Ib);
         }
+        sumM = radd2(sumM, L.Mb);  // (of the last stripe)
+        sumI = radd2(sumI, L.Ib);
     };
 
     for (int t0 = 0; t0 < steps; t0 += kChunk) {

@@ -235,11 +235,15 @@ constexpr double kUnflushedMin = 0x1p-700;
 
 // Sweep one stripe over the column stream of haplotypes [g_lo, g_hi): as `sweep` (phmm_device.cuh),
 // the scratch row holding the handed-on (I, sum) pair per column.  LR: LaneRowsEq or LaneRowsRow.
-template <int K, int V, bool FROM_SCR, bool TO_SCR, bool FLUSH, typename LR>
+// MULTI, from_scr, to_scr: as in the FP32 sweep (phmm_device2.cuh), one sweep for first, middle and last
+// stripes.
+template <int K, int V, bool MULTI, bool FLUSH, typename LR>
 __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTables<double>& tb,
                          const SweepOut& so, uint32_t g_lo, uint32_t g_hi, double* scr, int lane, bool above_row0,
-                         bool exotic, uint64_t roff, int R, int row0, uint32_t& again_lo, uint32_t& again_hi)
+                         bool exotic, uint64_t roff, int R, int row0, bool from_scr, bool to_scr, uint32_t& again_lo,
+                         uint32_t& again_hi)
 {
+    const bool FROM_SCR = MULTI && from_scr, TO_SCR = MULTI && to_scr;
     const uint64_t s0 = b.hap_off[g_lo];
     const int Tcols = (int)(b.hap_off[g_hi] - s0);
     const uint32_t* codes = (V == kInter ? b.codes_inter : b.codes_intra) + kCodePad + s0;
@@ -258,7 +262,7 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
     // in shared memory, copied two blocks ahead, so that lane 0 does not wait for L2 in every step.
     // Lane 31 writes the same row 31 columns behind lane 0 (for the stripe below), never a column still
     // to be read.
-    static_assert(!FROM_SCR || K == kMaxK, "the ring is part of the multi-stripe shape's table");
+    static_assert(!MULTI || K == kMaxK, "the ring is part of the multi-stripe shape's table");
     double* ring = tab + kTabClasses * K * kWarp;
     auto copy_block = [&](int c0) {
         if (lane < kScrBlock64 && c0 + lane < Tcols) {
@@ -317,14 +321,13 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
         double uS = shfl_up1(L.Sn);
         if (check && p == nb) boundary();
         if (lane == 0) {
+            // below the boundary row: I = fma(0, xx, 0 * mx) = 0
+            uI = 0.0;
+            uS = Stop;
             if (FROM_SCR) {
                 const bool ok = p >= 0 && p < Tcols;
                 uI = ok ? ring[2 * (p & (kScrRing64 - 1)) + 0] : 0.0;
                 uS = ok ? ring[2 * (p & (kScrRing64 - 1)) + 1] : 0.0;
-            } else {
-                // below the boundary row: I = fma(0, xx, 0 * mx) = 0
-                uI = 0.0;
-                uS = Stop;
             }
         }
         const uint32_t w = wn;
@@ -347,10 +350,9 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
                 scr[2 * p + 0] = L.In;
                 scr[2 * p + 1] = L.Sn;
             }
-        } else {
-            sumM = radd(sumM, L.Mb);
-            sumI = radd(sumI, L.Ib);
         }
+        sumM = radd(sumM, L.Mb);  // (of the last stripe)
+        sumI = radd(sumI, L.Ib);
     };
     static_assert(kScrBlock64 % kChunkScalar == 0, "a block of the ring is whole chunks");
 

@@ -43,19 +43,14 @@ __device__ __forceinline__ void run_pair2(const BatchView& b, const ProbTables<f
     const bool aboveX = lane * KH <= rp.pad[0], aboveY = lane * KH <= rp.pad[1];
     if (!MULTI) {
         const bool exotic = __any_sync(0xffffffffu, load_rows2<KH, V, PM>(L, tab, b, tb, rp, 0, lane));
-        sweep2<KH, V, PM, false, false>(L, tab, b, tb, pc, so, rp, 0, g_lo, g_hi, scr, lane, aboveX, aboveY, exotic);
+        sweep2<KH, V, PM, false>(L, tab, b, tb, pc, so, rp, 0, g_lo, g_hi, scr, lane, aboveX, aboveY, exotic, false,
+                                 false);
     } else {
         for (int s = 0; s < S; ++s) {
             const bool exotic = __any_sync(0xffffffffu, load_rows2<KH, V, PM>(L, tab, b, tb, rp, s * SR, lane));
             const bool aX = s == 0 && aboveX, aY = s == 0 && aboveY;
-            if (s == 0)
-                sweep2<KH, V, PM, false, true>(L, tab, b, tb, pc, so, rp, 0, g_lo, g_hi, scr, lane, aX, aY, exotic);
-            else if (s == S - 1)
-                sweep2<KH, V, PM, true, false>(L, tab, b, tb, pc, so, rp, s * SR, g_lo, g_hi, scr, lane, aX, aY,
-                                               exotic);
-            else
-                sweep2<KH, V, PM, true, true>(L, tab, b, tb, pc, so, rp, s * SR, g_lo, g_hi, scr, lane, aX, aY,
-                                              exotic);
+            sweep2<KH, V, PM, true>(L, tab, b, tb, pc, so, rp, s * SR, g_lo, g_hi, scr, lane, aX, aY, exotic, s > 0,
+                                    s < S - 1);
             __syncwarp();  // lane 31's scratch row is read by lane 0 in the next stripe
         }
     }

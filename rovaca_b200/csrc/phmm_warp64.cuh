@@ -35,18 +35,8 @@ __device__ __forceinline__ void run_stripes(const BatchView& b, const ProbTables
             exotic = load_rows_row<K, V>(L, tab, b, tb, roff, R, s * SR, pad, lane);
         const bool above_row0 = (s == 0) && (lane * K <= pad);
         const int row0 = s * SR - pad;  // read position of slot 0 of lane 0
-        if constexpr (!MULTI)
-            sweep_eq<K, V, false, false, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R,
-                                                row0, again_lo, again_hi);
-        else if (s == 0)
-            sweep_eq<K, V, false, true, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R,
-                                               row0, again_lo, again_hi);
-        else if (s == stripes - 1)
-            sweep_eq<K, V, true, false, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R,
-                                               row0, again_lo, again_hi);
-        else
-            sweep_eq<K, V, true, true, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R,
-                                              row0, again_lo, again_hi);
+        sweep_eq<K, V, MULTI, FLUSH>(L, tab, b, tb, so, g_lo, g_hi, scr, lane, above_row0, exotic, roff, R, row0, s > 0,
+                                     s < stripes - 1, again_lo, again_hi);
         // lane 31's scratch row is read by lane 0 in the next stripe; every lane's priors are rewritten
         __syncwarp();
     }
