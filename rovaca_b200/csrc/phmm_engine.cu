@@ -1142,26 +1142,24 @@ struct ChunkRange {
     uint64_t hap0, read0, out0;
 };
 
-// Cuts a validated batch at region boundaries near these cumulative shares of its cells: a small
-// first chunk gets the device going after little planning and uploading, and the rest is planned
-// and uploaded while it runs.  Measured on B200 over the 2,000-region benchmark batch end to end:
-// one cut at 15% 2278 GCUPS, one pipeline 2213; cuts at 10% and 55% 2238 and at 12.5%, 42% and 71%
-// 2237, their extra chunk tails adding 7-8 ms of device time.  With the current kernels: one cut
-// 2713 GCUPS, cuts at 15% and 85% 2682, and either with the serving slots' overlap scheduling on the
-// two chunk slots 2712 and 2717 (within noise); later, one cut at 15% 199.3-199.5 ms per batch, at 8%
-// 198.2-199.0, at 5% 197.9-198.4, at 3% 201.6-202.1 (the first chunk then ends before the second is
-// planned and uploaded) and at 22% 199.8.  The default (build-time setting) is 8%.
-std::vector<ChunkRange> split_chunks(const phmm_batch& b, uint64_t total_cells)
+// Cuts a validated batch in two at the region boundary near a share of its cells: a small first chunk gets
+// the device going after little planning and uploading, and the rest is planned and uploaded while it
+// runs, so its share follows the batch's bytes per cell (kFirstCellsPerByte cells of the first chunk per
+// byte of the batch, 5% to 20% of the cells).  Measured on B200 end to end, first chunk at 8% and 15%:
+// 1,000 benchmark regions (8.0e-4 bytes per cell) 104.1 and 105.4 ms, 150 regions with per-base gaps (8.4e-4)
+// 20.5 and 21.1, 60 low-quality regions (3.6e-4) 37.6 and 38.1, 1,500 regions at whole-genome depth (1.2e-3)
+// 23.7-24.2 and 22.3.  Two cuts (at 4% and 20%, 6% and 30%, 10% and 40%) cost 1,000 regions 4-6 ms more
+// than one at 8%.
+constexpr double kFirstCellsPerByte = 110.0;
+
+std::vector<ChunkRange> split_chunks(const phmm_batch& b, const BatchScan& sc)
 {
-#ifndef PHMM_CHUNK_FIRST
-#define PHMM_CHUNK_FIRST 0.08
-#endif
-    static const double kEnds[] = {PHMM_CHUNK_FIRST};
-    constexpr int kCuts = (int)(sizeof(kEnds) / sizeof(kEnds[0]));
+    const uint64_t total_cells = sc.cells;
+    const double bytes = 5.0 * (double)sc.read_bases + (double)sc.hap_bases;
+    const double cut = std::min(0.2, std::max(0.05, kFirstCellsPerByte * bytes / (double)std::max<uint64_t>(total_cells, 1)));
     std::vector<ChunkRange> ch;
     ChunkRange cur{0, 0, 0, 0, 0};
     uint64_t h = 0, r = 0, o = 0, cells = 0;
-    int next = 0;
     for (uint32_t g = 0; g < b.n_regions; ++g) {
         const uint32_t nh = b.n_haps[g], nr = b.n_reads[g];
         cells += (b.hap_off[h + nh] - b.hap_off[h]) * (b.read_off[r + nr] - b.read_off[r]);
@@ -1169,10 +1167,9 @@ std::vector<ChunkRange> split_chunks(const phmm_batch& b, uint64_t total_cells)
         r += nr;
         o += (uint64_t)nh * nr;
         cur.r1 = g + 1;
-        if (next < kCuts && (double)cells >= kEnds[next] * (double)total_cells && g + 1 < b.n_regions) {
+        if (ch.empty() && (double)cells >= cut * (double)total_cells && g + 1 < b.n_regions) {
             ch.push_back(cur);
             cur = ChunkRange{g + 1, g + 1, h, r, o};
-            while (next < kCuts && (double)cells >= kEnds[next] * (double)total_cells) ++next;
         }
     }
     if (cur.r1 > cur.r0) ch.push_back(cur);
@@ -1196,7 +1193,7 @@ phmm_status Engine::compute_chunked(const phmm_batch& b, const BatchScan& sc, do
                                     phmm_stats* stats, std::string& err, bool* ran)
 {
     *ran = false;
-    const std::vector<ChunkRange> ch = split_chunks(b, sc.cells);
+    const std::vector<ChunkRange> ch = split_chunks(b, sc);
     if (ch.size() < 2) return PHMM_OK;
     phmm_status st = PHMM_OK;
     if (!chunk_slot_) {
