@@ -73,7 +73,7 @@ typedef struct phmm_config {
     uint64_t chunk_cells;      /* phmm_compute_regions runs a batch of at least this many cells as a
                                   pipeline of region chunks on two device slots, planning and
                                   uploading each chunk while the previous one runs (same results);
-                                  0 = 4e10, UINT64_MAX = never */
+                                  0 = 2e9, UINT64_MAX = never */
 } phmm_config;
 
 /* A batch of independent active regions in flat, concatenated arrays (host memory). */

@@ -49,9 +49,11 @@ namespace {
 size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
 constexpr size_t kDescBytes = sizeof(BatchDesc) + sizeof(ClassDesc) * kNumClasses + 4 * sizeof(unsigned int);
-// Default phmm_config.chunk_cells: a batch of this many cells keeps the device busy for about 17 ms,
-// several times what planning and uploading its first chunk take.
-constexpr uint64_t kDefaultChunkCells = 40000000000ull;
+// Default phmm_config.chunk_cells: from here on (under 1 ms of device work) planning and uploading a batch
+// takes long enough to be worth hiding.  Measured on B200, one pipeline and two chunks, end to end: 2.4e9
+// cells (60 regions at whole-genome depth) 1.27 and 1.14 ms, 4.3e9 (20 benchmark regions) 2.55 and 2.35,
+// 9e9 4.05 and 3.5, 2e10 9.0 and 8.2, 4.4e10 17.2 and 16.4; 9.8e8 cells 0.89 either way.
+constexpr uint64_t kDefaultChunkCells = 2000000000ull;
 // Batches of fewer cells (about 8 ms of device work) launch their non-empty classes directly, with grids
 // cut to their items, instead of replaying the captured graph of all 66 classes at full grids, whose
 // empty launches alone take 0.2-0.4 ms.  Measured on B200, graph then direct, end to end: one region of
@@ -1144,19 +1146,20 @@ struct ChunkRange {
 
 // Cuts a validated batch in two at the region boundary near a share of its cells: a small first chunk gets
 // the device going after little planning and uploading, and the rest is planned and uploaded while it
-// runs, so its share follows the batch's bytes per cell (kFirstCellsPerByte cells of the first chunk per
-// byte of the batch, 5% to 20% of the cells).  Measured on B200 end to end, first chunk at 8% and 15%:
-// 1,000 benchmark regions (8.0e-4 bytes per cell) 104.1 and 105.4 ms, 150 regions with per-base gaps (8.4e-4)
-// 20.5 and 21.1, 60 low-quality regions (3.6e-4) 37.6 and 38.1, 1,500 regions at whole-genome depth (1.2e-3)
-// 23.7-24.2 and 22.3.  Two cuts (at 4% and 20%, 6% and 30%, 10% and 40%) cost 1,000 regions 4-6 ms more
-// than one at 8%.
-constexpr double kFirstCellsPerByte = 110.0;
+// runs, so its share (5% to 25% of the cells) follows the batch's bytes per cell, kFirstCellsPerByte cells
+// per byte of the batch, and a fixed cost of kFirstCells.  Measured on B200 end to end, in ms, at 110 and
+// 200 cells per byte: 1,000 benchmark regions (8.0e-4 bytes per cell) 102.8 and 103.5, 150 regions with
+// per-base gaps (8.4e-4) 20.5 and 20.7, 1,500 regions at whole-genome depth (1.2e-3) 22.9 and 22.0, 200 of
+// them 3.6 and 3.5, 20 benchmark regions 2.55 and 2.35.  Two cuts (at 4% and 20%, 6% and 30%, 10% and 40%)
+// cost 1,000 regions 4-6 ms more than one at 8%.
+constexpr double kFirstCellsPerByte = 130.0, kFirstCells = 6e8;
 
 std::vector<ChunkRange> split_chunks(const phmm_batch& b, const BatchScan& sc)
 {
     const uint64_t total_cells = sc.cells;
     const double bytes = 5.0 * (double)sc.read_bases + (double)sc.hap_bases;
-    const double cut = std::min(0.2, std::max(0.05, kFirstCellsPerByte * bytes / (double)std::max<uint64_t>(total_cells, 1)));
+    const double first = kFirstCellsPerByte * bytes + kFirstCells;
+    const double cut = std::min(0.25, std::max(0.05, first / (double)std::max<uint64_t>(total_cells, 1)));
     std::vector<ChunkRange> ch;
     ChunkRange cur{0, 0, 0, 0, 0};
     uint64_t h = 0, r = 0, o = 0, cells = 0;
