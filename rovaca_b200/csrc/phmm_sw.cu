@@ -33,6 +33,7 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -635,13 +636,20 @@ void staged_copy(void* dst, const void* src, size_t bytes)
         return;
     }
     const size_t part = (bytes + nt - 1) / nt;
-    std::vector<std::thread> pool;
+    auto copy = [=](size_t o) {
+        if (o < bytes) std::memcpy((char*)dst + o, (const char*)src + o, std::min(part, bytes - o));
+    };
+    std::thread pool[8];
     for (unsigned t = 1; t < nt; ++t) {
-        const size_t o = (size_t)t * part;
-        if (o < bytes) pool.emplace_back([=] { std::memcpy((char*)dst + o, (const char*)src + o, std::min(part, bytes - o)); });
+        try {
+            pool[t] = std::thread(copy, (size_t)t * part);
+        } catch (const std::system_error&) {  // no more threads: copy it here
+            copy((size_t)t * part);
+        }
     }
-    std::memcpy(dst, src, std::min(part, bytes));
-    for (auto& th : pool) th.join();
+    copy(0);
+    for (auto& th : pool)
+        if (th.joinable()) th.join();
 }
 
 phmm_status check_items(uint32_t n, const SwItem* items, uint64_t hap_bytes, uint64_t read_bytes, std::string& err)
@@ -999,7 +1007,7 @@ phmm_status SwAligner::align(const SwParams& prm, int variant, uint32_t n, const
     st = ensure_pinned(in.in_bytes(), err);
     if (st != PHMM_OK) return st;
     uint8_t* h = (uint8_t*)pinned_;
-    auto stage = [&] {
+    auto stage = [&]() noexcept {
         staged_copy(h + in.items, items, sizeof(SwItem) * (size_t)n);
         if (hap_bytes) staged_copy(h + in.hap, hap, hap_bytes);
         if (read_bytes) staged_copy(h + in.read, read, read_bytes);
@@ -1007,8 +1015,15 @@ phmm_status SwAligner::align(const SwParams& prm, int variant, uint32_t n, const
     SwPlan p;
     {
         std::thread helper;
-        if (hap_bytes + read_bytes >= (1u << 20)) helper = std::thread(stage);
-        else stage();
+        if (hap_bytes + read_bytes >= (1u << 20)) {
+            try {
+                helper = std::thread(stage);
+            } catch (const std::system_error&) {
+                stage();
+            }
+        } else {
+            stage();
+        }
         try {
             st = plan(prm, variant, n, items, cigar_cap, p, err);
         } catch (...) {
