@@ -138,17 +138,23 @@ __device__ __forceinline__ void copies_wait_all()
 #endif
 }
 
-// Columns of the FP64 kernels' ring of the row above a stripe (one (I, sum) pair per column): three
-// blocks of kScrBlock64 columns, two complete (the steps of a block and the vote's look past its end)
-// and one being copied, in four blocks of slots.
+// Columns of the FP64 kernels' ring of the row above a stripe (one (I, sum) pair per column): blocks of
+// kScrBlock64 columns, the one of the current steps, the next one (complete before a block's first step)
+// and the one being copied; four blocks of slots, so that a column's slot is its index modulo the ring.
 constexpr int kScrBlock64 = 16, kScrRing64 = 4 * kScrBlock64;
 // A warp's prior table: [class][row slot][lane], kTabClasses * K * kWarp values (and, for K = 8, the only
-// multi-stripe shape, the ring of the row above).
+// multi-stripe shape, the ring of the row above, behind it).
 template <int K>
 __host__ __device__ constexpr int prior_table_size()
 {
     return kTabClasses * K * kWarp + (K == kMaxK ? 2 * kScrRing64 : 0);
 }
+// The table in shared memory: the ring is filled by 16-byte copies, so it starts on a 16-byte boundary.
+template <int K>
+struct alignas(16) PriorTable64 {
+    double v[prior_table_size<K>()];
+};
+static_assert(kTabClasses * kMaxK * kWarp * sizeof(double) % 16 == 0, "the ring is not 16-byte aligned in the table");
 template <int K>
 __device__ __forceinline__ int prior_slot(uint32_t cls, int k, int lane)
 {

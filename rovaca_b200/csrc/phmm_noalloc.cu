@@ -38,7 +38,7 @@ namespace {
 
 constexpr size_t kNoAllocBytes = 64ull << 20;
 constexpr int kNoAllocMultiWarps = 64;    // multi-stripe classes run on this many warps here
-constexpr unsigned int kMultiCols = 4096; // = PlanLimits::max_stream_multi
+constexpr unsigned int kMultiCols = PlanLimits().max_stream_multi;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 

@@ -49,6 +49,8 @@ struct PlanLimits {
     // the batch's gap-quality arrays are not read (the device writes them).
     const RegionApiParams* region_api = nullptr;
 };
+// a warp's scratch row (24 bytes a column) is read by 16-byte copies, so every row starts on 16 bytes
+static_assert(PlanLimits().max_stream_multi % 2 == 0, "scratch rows are not 16-byte aligned");
 
 struct Plan {
     uint32_t n_regions = 0, n_reads = 0, n_haps = 0;
