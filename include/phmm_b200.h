@@ -65,7 +65,8 @@ typedef struct phmm_engine phmm_engine;
 typedef struct phmm_config {
     int32_t device;            /* CUDA device ordinal */
     int32_t use_cuda_graph;    /* 1: replay the device-side batch pipeline of a large batch (2e10 cells
-                                  or more) from a captured CUDA graph; 0: always launch directly */
+                                  or more) from a captured CUDA graph; 2: of every batch; 0: always
+                                  launch directly */
     int32_t autotune;          /* 1: run the tile-shape autotuner at creation (once per device and
                                   process; later engines reuse its table); 0: default shapes */
     int32_t reserved0;

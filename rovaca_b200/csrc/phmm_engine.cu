@@ -838,7 +838,7 @@ void Engine::full_layout(Slot& s)
 bool Engine::upload_raw(Slot& s, const BatchScan& sc, const phmm_batch& b)
 {
     // (a batch that may fit the compact layout waits for its plan)
-    if (sc.cells < kDirectCells && 5 * sc.read_bases + sc.hap_bases <= kCompactBytes / 2) return false;
+    if (cfg_.use_cuda_graph != 2 && sc.cells < kDirectCells && 5 * sc.read_bases + sc.hap_bases <= kCompactBytes / 2) return false;
     if (s.dev) full_layout(s);
     if (!s.dev || sc.read_bases > s.cap.read_bases || sc.hap_bases > s.cap.hap_bases) return false;
     cudaStream_t m = s.main;
@@ -987,7 +987,10 @@ PlanLimits Engine::limits_for(const TileTable& t, const BatchScan& sc) const
     return l;
 }
 
-bool Engine::use_graph(const Plan& plan) const { return cfg_.use_cuda_graph && plan.cells >= kDirectCells; }
+bool Engine::use_graph(const Plan& plan) const
+{
+    return cfg_.use_cuda_graph == 2 || (cfg_.use_cuda_graph && plan.cells >= kDirectCells);
+}
 
 phmm_status Engine::ensure_graph(Slot& s, const Plan& plan, bool want_flags, std::string& err)
 {

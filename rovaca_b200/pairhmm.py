@@ -232,9 +232,10 @@ def class64(mode: int, read_len: int) -> int:
 class Engine:
     """One engine per CUDA device (phmm_engine_create)."""
 
-    def __init__(self, device: int = 0, use_cuda_graph: bool = True, autotune: bool = True,
+    def __init__(self, device: int = 0, use_cuda_graph: bool | int = True, autotune: bool = True,
                  hbm_budget_bytes: int = 0, chunk_cells: int = 0):
-        """chunk_cells: compute() runs batches of at least this many cells as a pipeline of region
+        """use_cuda_graph: replay large batches from a captured graph (2: every batch, False: none).
+        chunk_cells: compute() runs batches of at least this many cells as a pipeline of region
         chunks (0: the library default, 2**64 - 1: never)."""
         self._lib = _lib.load()
         cfg = _lib.Config(device, int(use_cuda_graph), int(autotune), 0, hbm_budget_bytes, chunk_cells)
@@ -556,7 +557,7 @@ class DeviceSet:
     """One engine per listed device behind one handle (phmm_device_set_*): batches split across
     the devices by region, serving requests routed to the least-loaded device."""
 
-    def __init__(self, devices: Sequence[int], use_cuda_graph: bool = True, autotune: bool = True,
+    def __init__(self, devices: Sequence[int], use_cuda_graph: bool | int = True, autotune: bool = True,
                  hbm_budget_bytes: int = 0, chunk_cells: int = 0):
         self._lib = _lib.load()
         devs = (C.c_int32 * len(devices))(*devices)
