@@ -826,6 +826,7 @@ phmm_status Engine::capture_graph(Slot& s, bool want_flags, const TileTable& til
     }
     s.graph_flags = want_flags;
     s.graph_tiles = tiles;
+    s.graph_launches = s.launches;
     return PHMM_OK;
 }
 
@@ -1009,6 +1010,7 @@ phmm_status Engine::run(Slot& s, const Plan& plan, bool want_flags, bool restore
         st = ensure_graph(s, plan, want_flags, err);
         if (st != PHMM_OK) return st;
         PHMM_CK(cudaGraphLaunch(s.graph, m));
+        s.launches = s.graph_launches;
     } else {
         st = launch_pipeline(s, want_flags, &plan, plan.tiles, err);
         if (st != PHMM_OK) return st;

@@ -78,6 +78,7 @@ struct Slot {
     bool graph_flags = false;        // the captured graph writes pair flags
     TileTable graph_tiles{};         // tile table whose FP64 dependencies the graph encodes
     uint64_t launches = 0;           // kernels launched by the last pipeline run
+    uint64_t graph_launches = 0;     // kernels of the captured graph
     uint64_t arena_grows = 0;        // arena (re)allocations
     uint64_t graph_captures = 0;
     double setup_ms = 0.0;           // wall time spent growing the arena and capturing graphs

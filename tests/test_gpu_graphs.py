@@ -56,6 +56,24 @@ def test_a_graph_is_captured_again_for_a_new_tile_table(engine_direct):
                 _same(got, want)
 
 
+def test_large_batches_keep_their_graph_around_compact_ones(engine_direct):
+    """... and report its launches, not those of the direct launch before them."""
+    from rovaca_b200 import Engine
+
+    big, small = synth.config1(90, seed=21), synth.config1(1, seed=22)
+    want_big = engine_direct.compute(big, want_flags=True)
+    want_small = engine_direct.compute(small, want_flags=True)
+    assert want_big[2]["cells"] >= 2e10
+    with Engine(device=0, autotune=False, chunk_cells=2**64 - 1) as eng:
+        for step in ("big", "small", "big", "tiles", "big", "small", "small", "big"):
+            if step == "tiles":
+                eng.set_tiles(_table(lambda m, b: (5, 1) if b > 5 else None))
+                continue
+            got = eng.compute(big if step == "big" else small, want_flags=True)
+            assert (got[2]["kernel_launches"] > CLASSES) == (step == "big")
+            _same(got, want_big if step == "big" else want_small)
+
+
 def test_region_requests_through_the_graph_equal_direct_launches(engine):
     from rovaca_b200 import Engine
 
