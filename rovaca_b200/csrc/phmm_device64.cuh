@@ -231,7 +231,10 @@ __device__ __forceinline__ double row_diag(const LaneRowsRow<K>& L, int k, doubl
 // reads rarely pass: far from a read's alignment there are always values around 2^-1022.  Measured on
 // B200, FP64 pass of 24 regions of reads of 257-768 bases 6.2 ms then, 3.0 ms now; of 60 low-quality regions
 // 25.1 and 22.6 ms.
-constexpr double kUnflushedMin = 0x1p-700;
+#ifndef PHMM_F64_UNFLUSHED_MIN
+#define PHMM_F64_UNFLUSHED_MIN 0x1p-700  // (a test builds the CPU emulator with 0: no pair is swept again)
+#endif
+constexpr double kUnflushedMin = PHMM_F64_UNFLUSHED_MIN;
 
 // Sweep one stripe over the column stream of haplotypes [g_lo, g_hi): as `sweep` (phmm_device.cuh),
 // the scratch row holding the handed-on (I, sum) pair per column.  LR: LaneRowsEq or LaneRowsRow.

@@ -42,13 +42,13 @@ bool read_vec(FILE* f, std::vector<T>& v, size_t n)
 }
 
 // one warp: 32 threads run fn(lane) in lockstep at every collective
-void run_warp(const std::function<void(int)>& fn)
+void run_warp(const std::function<void(int)>& fn, bool flush)
 {
     warp_emu::Warp w;
     std::vector<std::thread> lanes;
     for (int l = 0; l < 32; ++l)
         lanes.emplace_back([&, l] {
-            warp_emu::enter_lane(&w, l);
+            warp_emu::enter_lane(&w, l, flush);
             fn(l);
         });
     for (auto& t : lanes) t.join();
@@ -58,7 +58,7 @@ template <int KH, int V, int PM, bool MULTI>
 void f32_class(const BatchView& b, const ProbTables<float>& t, const PassControl& pc)
 {
     std::vector<float4> tab(tab_floats4<KH>() + kRingFloat4);
-    run_warp([&](int lane) { warp_items32<KH, V, PM, MULTI>(b, t, pc, tab.data(), lane, 0, 0xffffffffu); });
+    run_warp([&](int lane) { warp_items32<KH, V, PM, MULTI>(b, t, pc, tab.data(), lane, 0, 0xffffffffu); }, true);
 }
 
 template <int V, int PM>
@@ -85,7 +85,7 @@ template <int K, int V, int PM, bool MULTI, bool UNF>
 void f64_class(const BatchView& b, const ProbTables<double>& t, const PassControl& pc)
 {
     std::vector<double> tab(prior_table_size<K>());
-    run_warp([&](int lane) { warp_reruns64<K, V, PM, MULTI, UNF>(b, t, pc, tab.data(), lane, 0); });
+    run_warp([&](int lane) { warp_reruns64<K, V, PM, MULTI, UNF>(b, t, pc, tab.data(), lane, 0); }, false);
 }
 
 template <int V, int PM, bool UNF>

@@ -82,11 +82,14 @@ struct Warp {
 inline thread_local Warp* t_warp = nullptr;
 inline thread_local int t_lane = 0;
 
-inline void enter_lane(Warp* w, int lane)
+// flush: FTZ | DAZ, as -ftz=true compiles the FP32 kernels.  FP64 arithmetic on the GPU has no flush mode:
+// the FP64 kernels' lanes keep values below 2^-1022 unless the code flushes them.
+inline void enter_lane(Warp* w, int lane, bool flush = true)
 {
     t_warp = w;
     t_lane = lane;
-    _mm_setcsr(_mm_getcsr() | 0x8040);  // FTZ | DAZ
+    const unsigned int csr = _mm_getcsr() & ~0x8040u;
+    _mm_setcsr(flush ? csr | 0x8040u : csr);
 }
 
 template <typename T>
