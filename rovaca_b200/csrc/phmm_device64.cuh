@@ -235,16 +235,18 @@ __device__ __forceinline__ double row_diag(const LaneRowsRow<K>& L, int k, doubl
 #define PHMM_F64_UNFLUSHED_MIN 0x1p-700  // (a test builds the CPU emulator with 0: no pair is swept again)
 #endif
 constexpr double kUnflushedMin = PHMM_F64_UNFLUSHED_MIN;
+// What the unflushed sweep leaves as the likelihood of a pair to be swept again (no likelihood is above 0).
+__device__ __forceinline__ double sweep_again() { return __longlong_as_double(0x7ff0000000000000ll); }
 
 // Sweep one stripe over the column stream of haplotypes [g_lo, g_hi): as `sweep` (phmm_device.cuh),
 // the scratch row holding the handed-on (I, sum) pair per column.  LR: LaneRowsEq or LaneRowsRow.
 // MULTI, from_scr, to_scr: as in the FP32 sweep (phmm_device2.cuh), one sweep for first, middle and last
-// stripes.
+// stripes.  tiny (lane 31): counts the haplotypes whose sum is below kUnflushedMin; without FLUSH they get
+// sweep_again() for a likelihood.
 template <int K, int V, bool MULTI, bool FLUSH, typename LR>
 __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTables<double>& tb,
                          const SweepOut& so, uint32_t g_lo, uint32_t g_hi, double* scr, int lane, bool above_row0,
-                         bool exotic, uint64_t roff, int R, int row0, bool from_scr, bool to_scr, uint32_t& again_lo,
-                         uint32_t& again_hi)
+                         bool exotic, uint64_t roff, int R, int row0, bool from_scr, bool to_scr, uint32_t& tiny)
 {
     const bool FROM_SCR = MULTI && from_scr, TO_SCR = MULTI && to_scr;
     const uint64_t s0 = b.hap_off[g_lo];
@@ -282,14 +284,12 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
     auto boundary = [&]() {
         if (started) {
             if (!TO_SCR && lane == kWarp - 1) {
-                // sums of flushed non-negative values are 0 or normal: no flush needed
+                // (sums of flushed non-negative values are 0 or normal: no flush needed)
                 const double tot = radd(sumM, sumI);
                 const uint64_t oi = so.out_base + (uint64_t)(cur - g_lo) * so.out_stride;
-                so.out[oi] = log10(tot) - Scale<double>::log10_initial();
-                if (!FLUSH && !(tot >= kUnflushedMin)) {  // to be swept again (lane 31's range)
-                    if (again_lo == again_hi) again_lo = cur;
-                    again_hi = cur + 1;
-                }
+                const bool small = !(tot >= kUnflushedMin);
+                so.out[oi] = !FLUSH && small ? sweep_again() : log10(tot) - Scale<double>::log10_initial();
+                tiny += small;
             }
             ++cur;
         }
@@ -359,6 +359,9 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
     };
     static_assert(kScrBlock64 % kChunkScalar == 0, "a block of the ring is whole chunks");
 
+    // A flushed step is four times the instructions of an unflushed one (three integer operations behind
+    // every FP64 operation), and its loop is kept rolled: unrolled by four as the other the
+    // call took 61.5 instead of 54.8 ms (B200, 96,000 pairs below 2^-700, each swept both ways).
     for (int t0 = 0; t0 < steps; t0 += kChunkScalar) {
         if (FROM_SCR && t0 % kScrBlock64 == 0) {  // columns up to t0 + 2 blocks are complete from here
             copies_wait_all();
@@ -367,9 +370,10 @@ __device__ void sweep_eq(LR& L, double* tab, const BatchView& b, const ProbTable
         }
         const int nb31 = __shfl_sync(0xffffffffu, nb, kWarp - 1);
         if (nb31 >= t0 + kChunkScalar && t0 + kChunkScalar <= steps) {
-#pragma unroll
+#pragma unroll(FLUSH ? 1 : kChunkScalar)
             for (int u = 0; u < kChunkScalar; ++u) step(t0 + u, false);
         } else {
+#pragma unroll 1
             for (int u = 0; u < kChunkScalar; ++u)
                 if (t0 + u < steps) step(t0 + u, true);
         }

@@ -53,26 +53,31 @@ __global__ void prep_kernel(const BatchDesc* __restrict__ desc, const uint8_t* _
 // claim, streamed through the read like an FP32 work item.
 // ------------------------------------------------------------------------------------------
 // Resident warps per SM of the FP64 classes of mode 0 (constant gaps, insertion = deletion), the
-// compiler's register bound: 16 (128 registers; 296 and 64 bytes of spill loads for 8 and 7 rows per lane).
-// Measured on B200 with the unflushed sweep, 8 rows: the FP64 pass of 60 low-quality regions 22.6 ms at 16
-// warps, 23.0 at 12, 23.6 at 11; of the 1,000-region batch 4.54 and 4.63 ms at 16 and 12; 7 rows 2.80 ms
-// at 16 and 2.87 at 12.  The other classes keep what they need.  Build-time settings.
+// compiler's register bound: 16 (128 registers; up to 200 bytes of spill loads) for 8 and 7 rows per lane in
+// one stripe, 12 (168 registers, no spills) for stripes.  Measured on B200 with the unflushed sweep, 8 rows:
+// the FP64 pass of 60 low-quality regions 22.6 ms at 16 warps, 23.0 at 12, 23.6 at 11; of the 1,000-region
+// batch 4.54 and 4.63 ms at 16 and 12; 7 rows 2.80 ms at 16 and 2.87 at 12; stripes: a call of 24 regions of
+// long reads 9.71 ms at 16 and 9.47 at 12, and of 11,520 pairs of foreign long reads, all swept with
+// flushes, 34.1 and 31.0 ms.  The other classes keep what they need.  Build-time settings.
 #ifndef PHMM_F64_MIN_WARPS_K8
 #define PHMM_F64_MIN_WARPS_K8 16
 #endif
 #ifndef PHMM_F64_MIN_WARPS_K7
 #define PHMM_F64_MIN_WARPS_K7 16
 #endif
-template <int K, int PM>
+#ifndef PHMM_F64_MIN_WARPS_MULTI
+#define PHMM_F64_MIN_WARPS_MULTI 12
+#endif
+template <int K, int PM, bool MULTI>
 constexpr int min_blocks64()
 {
-    return PM != PM_EQ ? 1 : K == 8 ? PHMM_F64_MIN_WARPS_K8 : K == 7 ? PHMM_F64_MIN_WARPS_K7 : 1;
+    return PM != PM_EQ ? 1 : MULTI ? PHMM_F64_MIN_WARPS_MULTI : K == 8 ? PHMM_F64_MIN_WARPS_K8 : K == 7 ? PHMM_F64_MIN_WARPS_K7 : 1;
 }
 
 // UNF: the all-FP64 check arithmetic (plain multiply and add), used to measure the error of every
 // likelihood; the recompute pass proper uses the reference's contracted arithmetic.
 template <int K, int V, int PM, bool MULTI, bool UNF = false>
-__global__ void __launch_bounds__(kFwdBlock, min_blocks64<K, PM>()) fwd_f64_kernel(BatchView b, ProbTables<double> tb, PassControl pc)
+__global__ void __launch_bounds__(kFwdBlock, min_blocks64<K, PM, MULTI>()) fwd_f64_kernel(BatchView b, ProbTables<double> tb, PassControl pc)
 {
     __shared__ PriorTable64<K> tab;
     const int lane = threadIdx.x & (kWarp - 1);

@@ -16,6 +16,7 @@
 //          read bases, qualities, insertion, deletion and gap-continuation qualities
 //   OUT    likelihoods [f64, out_total], pair flags [u8, out_total], status word [u32]
 //   MODE   engine (FP32 pass, then the FP64 recompute) | check64 (every pair, all-FP64 model)
+//          eq64, row64 (every pair through the FP64 recompute of mode 0, of modes 1 and 2)
 //   TILES  default | multi<KH> (read-length buckets above KH run in stripes of 32 KH rows)
 #include "warp_emu_shim.h"
 
@@ -273,5 +274,6 @@ int main(int argc, char** argv)
     fwrite(flags.data(), 1, flags.size(), o);
     fwrite(&status, 4, 1, o);
     std::fclose(o);
+    std::printf("collectives %llu\n", (unsigned long long)warp_emu::collectives.load());
     return 0;
 }

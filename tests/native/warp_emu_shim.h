@@ -4,9 +4,9 @@
 //
 // Arithmetic: every rounded intrinsic is one IEEE operation (the build passes -ffp-contract=off and
 // -mfma, so fmaf / fma are single fused instructions); packed float2 operations are two of them.
-// The GPU kernels run with flush-to-zero single precision (-ftz=true); each lane thread sets the
+// The FP32 kernels run with flush-to-zero single precision (-ftz=true): their lane threads set the
 // x86 FTZ and DAZ bits, which flush single-precision denormal results and inputs the same way.  The
-// FP64 path flushes explicitly (ftz in phmm_device.cuh), so the bits change no double result it keeps.
+// FP64 kernels' do not: the GPU has no FP64 flush mode, their code flushes explicitly.
 //
 // Warp collectives: each lane writes its value to a per-warp slot, all lanes meet at a barrier,
 // read the slot they need and meet again; the device code calls them on every lane in the same
@@ -51,6 +51,13 @@ inline int __double2hiint(double x)
     std::memcpy(&u, &x, 8);
     return (int)(uint32_t)(u >> 32);
 }
+inline double __longlong_as_double(long long u)
+{
+    double x;
+    std::memcpy(&x, &u, 8);
+    return x;
+}
+inline int __ffs(int x) { return __builtin_ffs(x); }
 inline unsigned int min(unsigned int a, unsigned int b) { return a < b ? a : b; }
 
 inline unsigned int atomicAdd(unsigned int* p, unsigned int v) { return __atomic_fetch_add(p, v, __ATOMIC_SEQ_CST); }
@@ -74,6 +81,8 @@ struct Barrier {
         }
     }
 };
+
+inline std::atomic<uint64_t> collectives{0};  // exchanges of all warps so far: what their steps cost
 
 struct Warp {
     Barrier bar;
@@ -112,6 +121,7 @@ template <typename T>
 inline T exchange(T v, int src)
 {
     Warp* w = t_warp;
+    if (t_lane == 0) collectives.fetch_add(1, std::memory_order_relaxed);
     w->slot[t_lane] = bits(v);
     w->bar.arrive_and_wait();
     const T r = from_bits<T>(w->slot[src]);
@@ -145,4 +155,5 @@ inline T __shfl_sync(unsigned, T v, int src)
 }
 inline int __any_sync(unsigned, int p) { return warp_emu::ballot(p != 0) != 0; }
 inline int __all_sync(unsigned, int p) { return warp_emu::ballot(p != 0) == 0xffffffffu; }
+inline uint32_t __ballot_sync(unsigned, int p) { return warp_emu::ballot(p != 0); }
 inline void __syncwarp() { warp_emu::t_warp->bar.arrive_and_wait(); }

@@ -13,7 +13,7 @@ import numpy as np
 import pytest
 
 from rovaca_b200.pairhmm import PackedBatch, Region
-from test_warp_emulator import CSRC, EXACT, LOG10_C_F64, NATIVE, _run, emulator  # noqa: F401
+from test_warp_emulator import CSRC, EXACT, LOG10_C_F64, NATIVE, _run, _write, emulator  # noqa: F401
 
 LINE = -700 * np.log10(2.0) - LOG10_C_F64  # the likelihood of a sum of 2^-700
 
@@ -80,6 +80,40 @@ def test_the_emulator_can_tell_the_second_sweep_left_out(oracle, tmp_path):
     wrong = _differs(got, want)
     assert status == 0 and wrong.any()
     assert not wrong[want >= LINE].any()  # above the line the unflushed sweep alone is enough
+
+
+def _collectives(binary, pb: PackedBatch, tmp_path) -> int:
+    """What the FP64 recompute of every pair of the batch cost: the collectives of its warps' steps."""
+    _write(pb, tmp_path / "batch.bin")
+    p = subprocess.run([str(binary), str(tmp_path / "batch.bin"), str(tmp_path / "out.bin"), "eq64", "default"],
+                       check=True, timeout=900, capture_output=True, text=True)
+    return int(p.stdout.split()[1])
+
+
+def _fit(order: str, reads: int = 1) -> PackedBatch:
+    """Haplotypes that hold the reads (g) and foreign ones (f), whose pairs are below the line."""
+    rng = np.random.default_rng(17)
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    own = acgt[rng.integers(0, 4, 160)]
+    foreign = np.frombuffer(b"ACGT", np.uint8)[3 - np.searchsorted(acgt, own)]  # no base of the reads' own place
+    haps = [(own if k == "g" else foreign).tobytes() for k in order]
+    gap = [bytes([80] * 160)] * reads
+    return PackedBatch.from_regions([Region(haps, [own.tobytes()] * reads, [bytes([60] * 160)] * reads, gap, gap, gap)])
+
+
+def test_only_the_haplotypes_below_the_line_are_swept_again(emulator, oracle, tmp_path):  # noqa: F811
+    """Foreign haplotypes at both ends of a run cost what the same ones next to each other cost, but for one
+    more fill of the wavefront (a fifth of a haplotype here): those between them are not swept again."""
+    want = _reference(oracle, _fit("fggggf"), 0)
+    assert (want[[0, 5]] < LINE).all() and (want[1:5] > LINE).all()
+    apart, together, none = (_collectives(emulator, _fit(o), tmp_path) for o in ("fggggf", "ffgggg", "gggggg"))
+    assert none < together < apart < 1.1 * together
+
+
+def test_runs_of_foreign_reads_are_not_all_swept_twice(emulator, tmp_path):  # noqa: F811
+    """Twelve runs whose pairs are all below the line: the first two are swept both ways."""
+    foreign, good = (_collectives(emulator, _fit(o, reads=12), tmp_path) for o in ("ff", "gg"))
+    assert 13 / 12 < foreign / good < 16 / 12
 
 
 def test_no_factor_of_the_cell_update_exceeds_one(oracle):
