@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <system_error>
 #include <thread>
 
 namespace phmm {
@@ -230,21 +231,45 @@ phmm_status build_plan(const phmm_batch& b, const PlanLimits& lim, Plan& plan, s
         plan.out_total = out_off;
     }
 
-    // Regions are planned independently on host threads: N flags, gap modes, read pairing,
-    // haplotype runs and work items, each counted per (FP32 class, stream-length bucket).
+    // Regions are planned independently on host threads: N flags, gap modes, read pairing and haplotype
+    // runs, the work items only counted per (FP32 class, stream-length bucket); the items are then written
+    // straight to their places.  (A batch has up to an item per read pair and haplotype, so what an item
+    // costs here shows in the calls of small and medium batches: written to a list first and sorted from
+    // there, 400 regions of 20 reads and 4 haplotypes took 696 us to plan instead of 349.)
     constexpr int kBuckets = 64;
     constexpr uint32_t kBucketCols = 128;
+    struct Group {  // reads of one region with one key, against the same runs
+        uint32_t region, key;
+        uint32_t read, n_reads;  // in Part::reads
+        uint32_t run, n_runs;    // in Part::runs
+    };
     struct Part {
-        std::vector<WorkItem> raw;
-        std::vector<uint32_t> key;
-        std::vector<uint32_t> count;
+        std::vector<Group> groups;
+        std::vector<uint32_t> reads;
+        std::vector<Run> runs;
+        std::vector<uint32_t> count;  // items per key; then, while they are written, the next one's place
         uint64_t rerun_cap[kClasses64] = {};
         uint64_t pairs = 0, cells = 0;
         uint32_t max_multi = 0;
     };
+    // a group's item for one run, but for its reads, and its sorting key (longest streams of a class first)
+    auto item_of = [](const Group& gr, const Run& run, uint32_t& skey) {
+        const bool uniform = ((gr.key >> 21) & 1) == 0, read_n = ((gr.key >> 22) & 1) != 0;
+        WorkItem it{};
+        it.region = gr.region;
+        it.hap_lo = run.lo;
+        it.hap_hi = run.hi;
+        it.kh = (uint8_t)(gr.key & 0xf);
+        it.stripes = (uint8_t)((gr.key >> 4) & 0xffff);
+        it.variant = read_n ? (uint8_t)kIntra : run.variant;
+        it.pmode = (it.variant == kInter && uniform) ? 0 : 1;
+        const int c32 = class32(it.variant, it.pmode, it.kh, ((gr.key >> 20) & 1) != 0);
+        skey = (uint32_t)c32 * kBuckets + (kBuckets - 1 - std::min<uint32_t>(run.cols / kBucketCols, kBuckets - 1));
+        return it;
+    };
     auto plan_range = [&](uint32_t g0, uint32_t g1, Part& part) {
         part.count.assign((size_t)kClasses32 * kBuckets, 0);
-        std::vector<Run> runs_split, runs_all, runs_split_m, runs_all_m;
+        std::vector<Run> runs;
         struct ReadKey {
             uint32_t key;  // (N, gap mode, multi, stripes, kh) packed; reads with equal keys share an item
             uint32_t read;
@@ -286,60 +311,73 @@ phmm_status build_plan(const phmm_batch& b, const PlanLimits& lim, Plan& plan, s
                               gr});
             }
             std::stable_sort(rk.begin(), rk.end(), [](const ReadKey& x, const ReadKey& y) { return x.key < y.key; });
-            bool runs_ready = false, runs_m_ready = false;
-            for (size_t k = 0; k < rk.size();) {
-                const uint32_t key = rk[k].key;
-                const uint32_t r0 = rk[k].read;
-                const uint32_t r1 = (k + 1 < rk.size() && rk[k + 1].key == key) ? rk[k + 1].read : kNoRead;
-                k += (r1 == kNoRead) ? 1 : 2;
-                const uint32_t kh = key & 0xf, stripes = (key >> 4) & 0xffff;
-                const bool uniform = ((key >> 21) & 1) == 0, read_n = ((key >> 22) & 1) != 0;
-                const bool multi = ((key >> 20) & 1) != 0;
-                const std::vector<Run>* runs;
-                if (!multi) {
-                    if (!runs_ready) {
-                        make_runs(hoff, hfl, M, lim.max_stream_single, true, runs_split);
-                        make_runs(hoff, hfl, M, lim.max_stream_single, false, runs_all);
-                        runs_ready = true;
-                    }
-                    runs = read_n ? &runs_all : &runs_split;
-                } else {
-                    if (!runs_m_ready) {
-                        make_runs(hoff, hfl, M, lim.max_stream_multi, true, runs_split_m);
-                        make_runs(hoff, hfl, M, lim.max_stream_multi, false, runs_all_m);
-                        runs_m_ready = true;
-                    }
-                    runs = read_n ? &runs_all_m : &runs_split_m;
+            // the region's runs, for single- and multi-stripe reads without and with an N, once needed
+            uint32_t run_at[4], run_n[4] = {}, next = 0;
+            for (size_t k = 0; k < rk.size(); k = next) {
+                Group gr{};
+                gr.region = g;
+                gr.key = rk[k].key;
+                gr.read = (uint32_t)part.reads.size();
+                for (next = (uint32_t)k; next < rk.size() && rk[next].key == gr.key; ++next) part.reads.push_back(rk[next].read);
+                gr.n_reads = next - (uint32_t)k;
+                const bool read_n = ((gr.key >> 22) & 1) != 0, multi = ((gr.key >> 20) & 1) != 0;
+                const int which = (multi ? 2 : 0) + (read_n ? 1 : 0);
+                if (run_n[which] == 0) {
+                    make_runs(hoff, hfl, M, multi ? lim.max_stream_multi : lim.max_stream_single, !read_n, runs);
+                    run_at[which] = (uint32_t)part.runs.size();
+                    run_n[which] = (uint32_t)runs.size();
+                    part.runs.insert(part.runs.end(), runs.begin(), runs.end());
                 }
-                const uint64_t R0 = plan.read_off[r0 + 1] - plan.read_off[r0];
-                const uint64_t R1 = r1 == kNoRead ? 0 : plan.read_off[r1 + 1] - plan.read_off[r1];
-                const uint64_t rows = R0 + R1;
-                const uint32_t nreads = r1 == kNoRead ? 1 : 2;
-                for (const Run& run : *runs) {
-                    WorkItem it{};
+                gr.run = run_at[which];
+                gr.n_runs = run_n[which];
+                if (gr.n_runs == 0) continue;
+                part.groups.push_back(gr);
+                // items, and haplotypes and columns of the runs per mode
+                uint64_t haps[kModes32] = {}, cols = 0, rows = 0;
+                for (uint32_t j = 0; j < gr.n_runs; ++j) {
+                    const Run& run = part.runs[gr.run + j];
+                    uint32_t skey;
+                    const WorkItem it = item_of(gr, run, skey);
+                    part.count[skey] += (gr.n_reads + 1) / 2;
+                    haps[mode32(it.variant, it.pmode)] += run.hi - run.lo;
+                    cols += run.cols;
+                    if (multi) part.max_multi = std::max(part.max_multi, run.cols);
+                }
+                // each read's pairs may go to the FP64 class of its own length
+                for (uint32_t q = 0; q < gr.n_reads; ++q) {
+                    const uint32_t r = part.reads[gr.read + q];
+                    const uint64_t R = plan.read_off[r + 1] - plan.read_off[r];
+                    rows += R;
+                    for (int m = 0; m < kModes32; ++m)
+                        if (haps[m]) {
+                            part.rerun_cap[class64_for_len(m, R)] += haps[m];
+                            part.pairs += haps[m];
+                        }
+                }
+                part.cells += cols * rows;
+            }
+        }
+    };
+    // the part's items: pairs of a group's reads in order, each against the group's runs in order
+    auto write_items = [&](Part& part) {
+        std::vector<WorkItem> tmpl;
+        std::vector<uint32_t*> place;
+        for (const Group& gr : part.groups) {
+            tmpl.resize(gr.n_runs);
+            place.resize(gr.n_runs);
+            for (uint32_t j = 0; j < gr.n_runs; ++j) {
+                uint32_t skey;
+                tmpl[j] = item_of(gr, part.runs[gr.run + j], skey);
+                place[j] = &part.count[skey];
+            }
+            const uint32_t* reads = part.reads.data() + gr.read;
+            for (uint32_t q = 0; q < gr.n_reads; q += 2) {
+                const uint32_t r0 = reads[q], r1 = q + 1 < gr.n_reads ? reads[q + 1] : kNoRead;
+                for (uint32_t j = 0; j < gr.n_runs; ++j) {
+                    WorkItem& it = plan.items[(*place[j])++];
+                    it = tmpl[j];
                     it.read[0] = r0;
                     it.read[1] = r1;
-                    it.region = g;
-                    it.hap_lo = run.lo;
-                    it.hap_hi = run.hi;
-                    it.kh = (uint8_t)kh;
-                    it.stripes = (uint8_t)stripes;
-                    it.variant = read_n ? (uint8_t)kIntra : run.variant;
-                    it.pmode = (it.variant == kInter && uniform) ? 0 : 1;
-                    const int c32 = class32(it.variant, it.pmode, (int)kh, multi);
-                    const uint32_t bucket = std::min<uint32_t>(run.cols / kBucketCols, kBuckets - 1);
-                    const uint32_t skey = (uint32_t)c32 * kBuckets + (kBuckets - 1 - bucket);  // longest first
-                    part.raw.push_back(it);
-                    part.key.push_back(skey);
-                    ++part.count[skey];
-                    const uint32_t npairs = nreads * (uint32_t)(run.hi - run.lo);
-                    // each read's pairs may go to the FP64 class of its own length
-                    const int m = mode32(it.variant, it.pmode);
-                    part.rerun_cap[class64_for_len(m, R0)] += run.hi - run.lo;
-                    if (r1 != kNoRead) part.rerun_cap[class64_for_len(m, R1)] += run.hi - run.lo;
-                    part.pairs += npairs;
-                    part.cells += (uint64_t)run.cols * rows;
-                    if (multi) part.max_multi = std::max(part.max_multi, run.cols);
                 }
             }
         }
@@ -348,6 +386,23 @@ phmm_status build_plan(const phmm_batch& b, const PlanLimits& lim, Plan& plan, s
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const unsigned nthreads = (unsigned)std::min<uint64_t>({hw, 32u, b.n_regions, work / (1u << 20) + 1});
     std::vector<Part> parts(nthreads);
+    // fn(part) for every part, on threads of their own (here, where no other can start)
+    auto for_parts = [&](bool threads, auto fn) {
+        std::vector<std::thread> pool;
+        pool.reserve(nthreads);
+        for (unsigned t2 = 1; t2 < nthreads; ++t2) {
+            if (threads) {
+                try {
+                    pool.emplace_back(fn, t2);
+                    continue;
+                } catch (const std::system_error&) {
+                }
+            }
+            fn(t2);
+        }
+        fn(0u);
+        for (auto& th : pool) th.join();
+    };
     {
         // contiguous region ranges with about equal bases each
         std::vector<uint32_t> cut(nthreads + 1, b.n_regions);
@@ -360,32 +415,30 @@ phmm_status build_plan(const phmm_batch& b, const PlanLimits& lim, Plan& plan, s
                    plan.hap_off[rd.hap_begin + rd.n_haps] - plan.hap_off[rd.hap_begin];
             if (acc * nthreads >= work * t) cut[t++] = g + 1;
         }
-        std::vector<std::thread> pool;
-        for (unsigned t2 = 1; t2 < nthreads; ++t2) pool.emplace_back(plan_range, cut[t2], cut[t2 + 1], std::ref(parts[t2]));
-        plan_range(cut[0], cut[1], parts[0]);
-        for (auto& th : pool) th.join();
+        for_parts(true, [&](unsigned t2) { plan_range(cut[t2], cut[t2 + 1], parts[t2]); });
     }
-    std::vector<uint32_t> count((size_t)kClasses32 * kBuckets, 0);
-    size_t n_items = 0;
+    // items in the order of their keys, those of one key in region order (a stable counting sort)
+    std::vector<uint32_t> start((size_t)kClasses32 * kBuckets + 1, 0);
+    for (size_t i = 0; i + 1 < start.size(); ++i) {
+        uint32_t at = start[i];
+        for (Part& p : parts) {
+            const uint32_t n = p.count[i];
+            p.count[i] = at;
+            at += n;
+        }
+        start[i + 1] = at;
+    }
+    const size_t n_items = start.back();
     for (const Part& p : parts) {
-        for (size_t i = 0; i < count.size(); ++i) count[i] += p.count[i];
         for (int c = 0; c < kClasses64; ++c) plan.classes[kClasses32 + c].rerun_cap += (uint32_t)p.rerun_cap[c];
         plan.pairs += p.pairs;
         plan.cells += p.cells;
         plan.max_multi_stream = std::max(plan.max_multi_stream, p.max_multi);
-        n_items += p.raw.size();
     }
     plan.empty_pairs = plan.out_total - plan.pairs;
-
-    // stable counting sort by key (parts in region order)
-    std::vector<uint32_t> start(count.size() + 1, 0);
-    for (size_t i = 0; i < count.size(); ++i) start[i + 1] = start[i] + count[i];
     plan.items.resize(n_items);
-    {
-        std::vector<uint32_t> pos(start.begin(), start.end() - 1);
-        for (const Part& p : parts)
-            for (size_t i = 0; i < p.raw.size(); ++i) plan.items[pos[p.key[i]]++] = p.raw[i];
-    }
+    // (a thread costs about as much as 10,000 items)
+    for_parts(n_items >= (1u << 16), [&](unsigned t2) { write_items(parts[t2]); });
     for (int c = 0; c < kClasses32; ++c) {
         ClassDesc& cd = plan.classes[c];
         cd.item_off = start[(size_t)c * kBuckets];
