@@ -392,11 +392,13 @@ phmm_status grow_pinned(char*& p, size_t& bytes, size_t need, std::string& err)
 phmm_status Engine::realign_enqueue(Slot& s, RealignBatch& rb, std::string& err)
 {
     if (rb.plan.n == 0) return PHMM_OK;
-    rb.layout();
     // growing frees the old buffers, which waits for the device: only this slot's work is queued
     // before the wait, and arenas stop growing once they cover the slot's largest batch
-    if (rb.bytes > s.rdev_bytes) PHMM_CK(cudaStreamSynchronize(s.main));
-    phmm_status st = grow_device(s.rdev, s.rdev_bytes, rb.bytes, err);
+    phmm_status st = sw_alloc(rb.plan, [&]() -> phmm_status {
+        rb.layout();
+        if (rb.bytes > s.rdev_bytes) PHMM_CK(cudaStreamSynchronize(s.main));
+        return grow_device(s.rdev, s.rdev_bytes, rb.bytes, err);
+    });
     if (st != PHMM_OK) return st;
     st = grow_pinned(s.rpin, s.rpin_bytes, std::max(rb.upload_bytes(), rb.head_bytes()), err);
     if (st != PHMM_OK) return st;

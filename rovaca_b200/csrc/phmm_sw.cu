@@ -765,7 +765,7 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
     for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
     p.order.assign(n, 0);
     for (uint32_t q = 0; q < n; ++q) p.order[start[key[q]]++] = q;
-    uint64_t need[kSwGroups] = {}, sum = 0, most = 0;
+    uint64_t sum = 0;
     for (int g = 0; g < kSwGroups; ++g) {
         const uint32_t m = counts[g];
         if (m == 0) continue;
@@ -790,18 +790,11 @@ phmm_status sw_plan(int device, const SwParams& prm, int variant, uint32_t n, co
         }
         blocks = std::min<uint64_t>(blocks, std::max<uint64_t>(1, kSwScratchCap / (warps * p.stride[g])));
         p.grid[g] = (int)blocks;
-        need[g] = blocks * warps * p.stride[g];
-        sum += need[g];
-        most = std::max(most, need[g]);
+        p.need[g] = blocks * warps * p.stride[g];
+        sum += p.need[g];
     }
     // the groups run side by side, each in scratch of its own, when all of it fits the bound
-    p.concurrent = sum <= kSwScratchCap;
-    p.scratch = p.concurrent ? sum : most;
-    uint64_t at = 0;
-    for (int g = 0; g < kSwGroups && p.concurrent; ++g) {
-        p.scratch_off[g] = at;
-        at += need[g];
-    }
+    p.lay_out(sum <= kSwScratchCap);
     p.gather_blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((n + 7) / 8, (uint64_t)di.sms * 8));
     return PHMM_OK;
 }
@@ -1050,22 +1043,27 @@ phmm_status SwAligner::align(const SwParams& prm, int variant, uint32_t n, const
     }
     if (failed) std::rethrow_exception(failed);
     if (st != PHMM_OK) return st;
-    const SwArenaLayout L(n, hap_bytes, read_bytes, p.slots, p.scratch);
-    if (L.bytes > arena_bytes_) {
+    st = sw_alloc(p, [&]() -> phmm_status {
+        const SwArenaLayout need(n, hap_bytes, read_bytes, p.slots, p.scratch);
+        if (need.bytes <= arena_bytes_) return PHMM_OK;
         if (arena_) {
             SW_CK(cudaStreamSynchronize(stream_));
             cudaFree(arena_);
             arena_ = nullptr;
             arena_bytes_ = 0;
         }
-        const uint64_t sz = L.bytes + L.bytes / 4;
+        const uint64_t sz = need.bytes + need.bytes / 4;
         if (cudaMalloc(&arena_, sz) != cudaSuccess) {
             cudaGetLastError();
+            arena_ = nullptr;
             err = "Smith-Waterman arena of " + std::to_string(sz) + " bytes could not be allocated";
             return PHMM_ERR_OUT_OF_MEMORY;
         }
         arena_bytes_ = sz;
-    }
+        return PHMM_OK;
+    });
+    if (st != PHMM_OK) return st;
+    const SwArenaLayout L(n, hap_bytes, read_bytes, p.slots, p.scratch);
     uint8_t* d = (uint8_t*)arena_;
     std::memcpy(h + L.order, p.order.data(), 4ull * n);
     std::memcpy(h + L.slot_off, p.slot_off.data(), 8ull * n);
@@ -1096,12 +1094,16 @@ phmm_status SwAligner::resident_create(const SwParams& prm, int variant, uint32_
         delete r;
         return st;
     }
-    r->lay = SwArenaLayout(n, hap_bytes, read_bytes, r->plan.slots, r->plan.scratch);
-    if (cudaMalloc(&r->arena, r->lay.bytes) != cudaSuccess) {
+    st = sw_alloc(r->plan, [&] {
+        r->lay = SwArenaLayout(n, hap_bytes, read_bytes, r->plan.slots, r->plan.scratch);
+        if (cudaMalloc(&r->arena, r->lay.bytes) == cudaSuccess) return PHMM_OK;
         cudaGetLastError();
         err = "Smith-Waterman resident arena of " + std::to_string(r->lay.bytes) + " bytes could not be allocated";
-        delete r;
         return PHMM_ERR_OUT_OF_MEMORY;
+    });
+    if (st != PHMM_OK) {
+        delete r;
+        return st;
     }
     r->d = (uint8_t*)r->arena;
     auto up = [&](uint64_t off, const void* src, uint64_t bytes) {

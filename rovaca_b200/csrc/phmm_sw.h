@@ -154,14 +154,42 @@ struct SwPlan {
     uint64_t slots = 0;                      // ops of all slots
     uint32_t begin[kSwGroups + 1] = {};
     uint64_t stride[kSwGroups] = {};         // scratch bytes per warp of each group
-    uint64_t scratch_off[kSwGroups] = {};    // its scratch
+    uint64_t need[kSwGroups] = {};           // scratch bytes of each group
+    uint64_t scratch_off[kSwGroups] = {};    // where they lie
     uint32_t max_rows[kSwGroups] = {};       // longest haplotype of the group (two-per-warp groups)
     int grid[kSwGroups] = {};
     bool concurrent = true;                  // the groups have disjoint scratch and may run together
     int gather_blocks = 1;
     uint64_t scratch = 0;                    // bytes of all of it
     uint64_t cells = 0;
+
+    // Disjoint scratch for every group, or one piece for all, which then run one after another.
+    void lay_out(bool side_by_side)
+    {
+        concurrent = side_by_side;
+        uint64_t at = 0, most = 0;
+        for (int g = 0; g < kSwGroups; ++g) {
+            scratch_off[g] = side_by_side ? at : 0;
+            at += need[g];
+            most = need[g] > most ? need[g] : most;
+        }
+        scratch = side_by_side ? at : most;
+    }
 };
+
+// alloc() finds room for a planned batch; when there is none for its groups side by side, again with the
+// scratch shared between them.
+template <typename Alloc>
+phmm_status sw_alloc(SwPlan& p, Alloc alloc)
+{
+    phmm_status st = alloc();
+    if (st == PHMM_ERR_OUT_OF_MEMORY && p.concurrent) {
+        const uint64_t before = p.scratch;
+        p.lay_out(false);
+        if (p.scratch < before) st = alloc();
+    }
+    return st;
+}
 
 // Device buffers of one batch (see SwPlan for their sizes: n items, n results, `slots` ops twice,
 // `scratch` bytes, kSwGroups claim counters).
