@@ -2,6 +2,7 @@
 // the batch into wavefront work items grouped by kernel class, longest first inside a class.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -90,6 +91,18 @@ struct BatchScan {
 // item the pass takes about (stream_cols (1 + o / c) / warps + c) steps, least at
 // c = sqrt(stream_cols o / warps).
 uint32_t run_cols_for(uint64_t stream_cols, uint64_t warps);
+
+// Device bytes a region takes in the arena of a batch, at most (the serving loop holds its batches to a
+// share of the memory budget by this): gap qualities and bases of the reads, haplotypes with their code
+// words, two likelihoods, a flag and a rerun slot per pair, the descriptors, and work items, of which a
+// small batch has up to one per read pair and haplotype.
+inline uint64_t region_bytes(uint64_t read_bases, uint64_t hap_bases, uint64_t pairs, uint64_t n_reads, uint64_t n_haps)
+{
+    // (reads pair within one of at most 96 kinds: with or without an N, constant gaps or not, 24 lengths)
+    const uint64_t items = (n_reads + std::min<uint64_t>(n_reads, 96) + 1) / 2 * n_haps;
+    return read_bases * 5 + hap_bases * 9 + pairs * (8 + 8 + 1 + sizeof(RerunEntry)) + items * sizeof(WorkItem) +
+           n_reads * 11 + n_haps * 9 + 4096;
+}
 
 // Validation shared by every entry point: counts, non-decreasing offsets, the reference limits and
 // the pointers the batch needs.  Returns PHMM_OK, PHMM_ERR_INVALID_ARGUMENT or

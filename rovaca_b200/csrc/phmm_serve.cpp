@@ -105,7 +105,8 @@ struct Request {
     std::string own_error;
     uint64_t out_n = 0;
     uint64_t cells = 0;
-    uint64_t bytes = 0;  // device footprint estimate for admission
+    uint64_t least = 0;  // the request is refused when this exceeds the budget
+    uint64_t bytes = 0;  // its share of a batch's arena, at most: what the batches are held to
     Clock::time_point t_submit, t_admit, t_done;
 };
 
@@ -184,7 +185,8 @@ void run_copies(const std::vector<HostCopy>& copies, size_t total)
     for (auto& h : helpers) h.join();
 }
 
-uint64_t footprint(uint64_t read_bases, uint64_t hap_bases, uint64_t pairs, uint64_t n_reads, uint64_t n_haps)
+// The least a request must leave of the budget to be accepted (a batch of long runs, results only).
+uint64_t least_bytes(uint64_t read_bases, uint64_t hap_bases, uint64_t pairs, uint64_t n_reads, uint64_t n_haps)
 {
     return read_bases * 5 + hap_bases * 9 + pairs * (8 + 1 + 16) + n_reads * 17 + n_haps * 9 + 4096;
 }
@@ -578,11 +580,12 @@ phmm_status enqueue_request(phmm_engine* engine, const std::shared_ptr<Request>&
                             std::string& err)
 {
     Server* s = server_for(engine, true);
-    if (r->bytes > s->budget) {
-        err = "region needs about " + std::to_string(r->bytes) + " device bytes, more than the HBM budget of " +
+    if (r->least > s->budget) {
+        err = "region needs about " + std::to_string(r->least) + " device bytes, more than the HBM budget of " +
               std::to_string(s->budget);
         return PHMM_ERR_LIMIT_EXCEEDED;
     }
+    r->bytes = std::min(std::max(r->bytes, r->least), s->budget);  // (an accepted request alone always fits)
     {
         std::lock_guard<std::mutex> lk(s->mu);
         if (s->stop) {
@@ -639,10 +642,12 @@ phmm_status server_submit(phmm_engine* engine, const phmm_batch& b, double* out,
     r->flags = flags;
     r->out_n = sc.out_total;
     r->cells = sc.cells;
-    r->bytes = footprint(sc.read_bases, sc.hap_bases, sc.out_total, sc.n_reads, sc.n_haps);
+    r->least = least_bytes(sc.read_bases, sc.hap_bases, sc.out_total, sc.n_reads, sc.n_haps);
+    r->bytes = region_bytes(sc.read_bases, sc.hap_bases, sc.out_total, sc.n_reads, sc.n_haps);
     // a read longer than one stripe needs the per-warp scratch rows
     for (uint32_t k = 0; k < sc.n_reads; ++k)
         if (r->read_off[k + 1] - r->read_off[k] > (uint64_t)kWarp * kMaxK) {
+            r->least += engine_of(engine)->scratch_bytes();
             r->bytes += engine_of(engine)->scratch_bytes();
             break;
         }
@@ -765,14 +770,21 @@ phmm_status server_submit_region(phmm_engine* engine, const phmm_region_input& i
     r->n_kept = n_kept;
     r->out_n = sc.out_total;
     r->cells = sc.cells;
-    r->bytes = footprint(sc.read_bases, sc.hap_bases, sc.out_total, sc.n_reads, sc.n_haps) + sc.out_total * 8 +
-               sc.n_reads * 2 + r->hap_allele.size() + (r->gl_n + r->allele_lk_n) * 8 + n_events * 36;
-    if (r->realign)  // items, results and two CIGAR slots per read, and its share of the scratch
-        r->bytes += sc.n_reads * (96 + 8ull * std::min<uint64_t>(kSwMaxSeq - 1, r->max_hap + (sc.read_bases /
-                                                                        std::max<uint32_t>(sc.n_reads, 1) + 1)))
-                    + sc.read_bases * (r->max_hap / 2 + 64) + 4096;
+    const uint64_t events_bytes = r->hap_allele.size() + (r->gl_n + r->allele_lk_n) * 8 + n_events * 36;
+    r->least = least_bytes(sc.read_bases, sc.hap_bases, sc.out_total, sc.n_reads, sc.n_haps) + sc.out_total * 8 +
+               sc.n_reads * 2 + events_bytes;
+    r->bytes = region_bytes(sc.read_bases, sc.hap_bases, sc.out_total, sc.n_reads, sc.n_haps) + events_bytes;
+    if (r->realign) {  // items, results and two CIGAR slots per read, and its share of the scratch
+        const uint64_t mean = sc.read_bases / std::max<uint32_t>(sc.n_reads, 1) + 1;
+        const uint64_t items = sc.n_reads * (96 + 8ull * std::min<uint64_t>(kSwMaxSeq - 1, r->max_hap + mean)) + 4096;
+        r->least += items + sc.read_bases * (r->max_hap / 2 + 64);
+        r->bytes += items + realign_scratch_bytes(r->max_hap, sc.n_reads, [&](uint32_t k) {
+                        return (uint32_t)(r->read_off[k + 1] - r->read_off[k] - r->clip[2 * k] - r->clip[2 * k + 1]);
+                    });
+    }
     for (uint32_t k = 0; k < sc.n_reads; ++k)
         if (r->read_off[k + 1] - r->read_off[k] > (uint64_t)kWarp * kMaxK) {
+            r->least += engine_of(engine)->scratch_bytes();
             r->bytes += engine_of(engine)->scratch_bytes();
             break;
         }

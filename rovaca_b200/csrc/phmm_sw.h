@@ -142,6 +142,40 @@ inline SwForm sw_form(const SwParams& p, bool i32, uint32_t nrow, uint32_t ncol,
     return reach <= 32000 ? kSwRebased16 : kSwOnePerWarp;
 }
 
+// Device scratch of one two-per-warp warp (phmm_sw16.cuh): the cells' codes [steps][ceil(K/4)][32] u32, then
+// the runs of X and of Y.  A step's codes are one row: the lanes work on different haplotype rows then, and
+// a layout by haplotype row would scatter every store over 32 lines (K = 7: 1.60 ms against 0.76 for the
+// 15,000 alignments of 300 regions, the stores the bound).
+struct Sw16Layout {
+    uint64_t runs, run_stride, total;
+};
+PHMM_HD inline Sw16Layout sw16_layout(uint32_t max_rows, int K)
+{
+    Sw16Layout L;
+    const uint64_t nw = (uint64_t)(K + 3) / 4;
+    L.runs = sw_align256((uint64_t)(max_rows + 31) * 32 * nw * 4);
+    L.run_stride = sw_align256(4ull * (max_rows + 32ull * K + 4));
+    L.total = L.runs + 2 * L.run_stride;
+    return L;
+}
+
+// Scratch that realigning a region's n clipped reads (col(q) bases each) to haplotypes of at most `rows`
+// bases takes by itself, at most: every two of one stripe width in one warp.
+template <typename Col>
+uint64_t realign_scratch_bytes(uint32_t rows, uint32_t n, Col col)
+{
+    uint32_t count[kSwWrapClass] = {};
+    for (uint32_t q = 0; q < n; ++q) {
+        int c = 0;
+        while (c + 1 < kSwWrapClass && 32u * (uint32_t)kSwK[c] < col(q)) ++c;
+        ++count[c];
+    }
+    uint64_t bytes = 0;
+    for (int c = 0; c < kSwWrapClass; ++c)
+        if (count[c]) bytes += ((uint64_t)count[c] + 1) / 2 * sw16_layout(rows, kSwK[c]).total;
+    return bytes;
+}
+
 int sw_class_of(const SwParams& prm, int variant, uint32_t nrow, uint32_t ncol);
 
 // Host plan of one batch of alignments: launch group of each (by read columns and parameters),

@@ -106,22 +106,6 @@ struct Sw16Shared {
     PHMM_HD static uint32_t bytes(uint32_t max_rows) { return (rows_off(max_rows) + (max_rows + 64) * 2 + 15) & ~15u; }
 };
 
-// Device scratch of one warp: the cells' codes [steps][ceil(K/4)][32] u32, then the runs of X and of Y.
-// A step's codes are one row: the lanes work on different haplotype rows then, and a layout by haplotype
-// row would scatter every store over 32 lines (K = 7: 1.60 ms against 0.76 for the 15,000 alignments of 300 regions, the stores the bound).
-struct Sw16Layout {
-    uint64_t runs, run_stride, total;
-};
-PHMM_HD inline Sw16Layout sw16_layout(uint32_t max_rows, int K)
-{
-    Sw16Layout L;
-    const uint64_t nw = (uint64_t)(K + 3) / 4;
-    L.runs = sw_align256((uint64_t)(max_rows + 31) * 32 * nw * 4);
-    L.run_stride = sw_align256(4ull * (max_rows + 32ull * K + 4));
-    L.total = L.runs + 2 * L.run_stride;
-    return L;
-}
-
 struct Sw16Half {
     const uint8_t* hap;
     const uint8_t* read;
