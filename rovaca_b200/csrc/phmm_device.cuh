@@ -37,11 +37,10 @@
 
 namespace phmm {
 
-// Steps per boundary-free chunk of the scalar sweep (the FP64 recompute), a build-time setting:
-// the double-precision cell update is about twice the code of the FP32 one, so the unrolled chunk
-// decides how much of the hot loop the instruction cache has to hold.  Measured on B200 over the
-// 2,000-region benchmark batch: chunks of 2 or 4 steps cut the FP64 tail from 54 to 39 ms against
-// 8 steps (instruction-fetch stalls), 4 being marginally the best.
+// Steps per boundary-free chunk of the scalar sweeps (FP64), a build-time setting: the double-precision
+// cell update is about twice the code of the FP32 one, so the unrolled chunk decides how much of the hot
+// loop the instruction cache has to hold.  Measured on B200, FP64 pass of 60 low-quality regions: chunks of
+// 2 steps 24.0 ms, 4 steps 23.0, 8 steps 22.6 but 19% more on long reads, 16 steps 25.5.
 #ifndef PHMM_CHUNK_SCALAR
 #define PHMM_CHUNK_SCALAR 4
 #endif
@@ -56,8 +55,8 @@ __device__ __forceinline__ double rfma(double a, double b, double c) { return __
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 
 // FP64 has no hardware flush-to-zero; the reference's MXCSR.FTZ flushes tiny double results, so
-// the FP64 path flushes explicitly.  Results below 2^-1022 only arise far below any likelihood
-// that survives the FP32 -> FP64 switch, so this only keeps the two paths identical.  Every value
+// the FP64 paths flush explicitly where that can change a likelihood (phmm_device64.cuh; the all-FP64
+// check in every step its vote does not clear).  Every value
 // of the recurrence is >= 0 (probabilities times a positive scale), so a double is subnormal or
 // zero exactly when its high word is below 0x00100000 (biased exponent 0): an integer compare and
 // two selects, with no FP64-pipe instruction (a DSETP would take one of the pipe's slots per flush,
@@ -263,29 +262,20 @@ __device__ __forceinline__ void cells(LaneRows<T, K, PM>& L, const T (&pr)[K], T
     }
 }
 
-// Smallest value every nonzero input of an FP64 step must reach for no result of that step to fall
-// below 2^-1022, so that the step may skip the flushes and still give the flushed results.  Every
-// nonzero probability of the tables is at least 2^-44 (the smallest, ph2pr(127) / 3, is 6.6e-14), all
-// values are >= 0, and a sum of non-negative terms is at least its largest term; the longest chain
-// of products in one step is the insertion recurrence down the lane's K rows (I(a) >= I(a-1) xx,
-// after M(a-1) = s prior and the product M mx), so every nonzero result is >= input x 2^(-44 (K+1)).
-// Expressed as the high word of that double (biased exponent 1023 - 1022 + 44 (K + 1)).
-#ifndef PHMM_F64_VOTE
-#define PHMM_F64_VOTE 1  // 0: every FP64 step flushes (no vote)
-#endif
+// The all-FP64 check kernels (the only sweep that votes) run a step without flushes where they could change
+// nothing: the smallest value every nonzero input of the next kVoteSteps steps must reach for no result of
+// theirs to fall below 2^-1022.  Every nonzero probability of the tables is at least 2^-44 (the smallest,
+// ph2pr(127) / 3, is 6.6e-14), all values are >= 0, and a sum of non-negative terms is at least its
+// largest term; the longest chain of products in one step is the insertion recurrence down the lane's K
+// rows (I(a) >= I(a-1) xx, after M(a-1) = s prior and the product M mx), so every nonzero result is
+// >= input x 2^(-44 (K+1)), and one of the step after >= input x 2^(-88 (K+1)).  Expressed as the high word
+// of that double (biased exponent 1023 - 1022 + 44 kVoteSteps (K + 1)).
+constexpr int kVoteSteps = 2;
 
-// Steps per vote: the bound then covers that many steps (an input of the second step is at least
-// the first step's inputs x 2^(-44 (K+1))).  Measured on B200: 2 cut the FP64 pass of the
-// underflow-stress shape from 56 to 50 ms against 1; 3 gained nothing more, and at 4 the bound
-// (2^562 for K = 8) is above most values, so nearly every step flushes.
-#ifndef PHMM_F64_VOTE_EVERY
-#define PHMM_F64_VOTE_EVERY 2
-#endif
-
-template <int K, int STEPS = PHMM_F64_VOTE_EVERY>
+template <int K>
 __device__ __forceinline__ uint32_t flush_free_hi()
 {
-    return (uint32_t)(1 + 44 * STEPS * (K + 1)) << 20;
+    return (uint32_t)(1 + 44 * kVoteSteps * (K + 1)) << 20;
 }
 
 // Whether every nonzero input of the lane's next step reaches flush_free_hi<K>(): its rows and the
@@ -410,9 +400,9 @@ __device__ void sweep(LaneRows<T, K, PM>& L, const T* tab, const BatchView& b, c
             }
         }
         // FP64: the flushes can only change a step whose inputs hold a value below the bound; the
-        // warp votes every PHMM_F64_VOTE_EVERY steps (the scratch row read by stripes after the first
-        // is not checked)
-        constexpr bool kVote = PHMM_F64_VOTE && sizeof(T) == 8 && !FROM_SCR;
+        // warp votes every kVoteSteps steps (the scratch row read by stripes after the first is not
+        // checked)
+        constexpr bool kVote = sizeof(T) == 8 && !FROM_SCR;
         if (kVote && flush_free)
             cells<T, K, V, PM, false, UNF>(L, pr, sM, sI, dM, dI, dD);
         else
@@ -431,7 +421,7 @@ __device__ void sweep(LaneRows<T, K, PM>& L, const T* tab, const BatchView& b, c
             sumI = radd(sumI, L.Ip[K - 1]);
         }
         if constexpr (kVote)
-            if (PHMM_F64_VOTE_EVERY == 1 || t % PHMM_F64_VOTE_EVERY == PHMM_F64_VOTE_EVERY - 1)
+            if (t % kVoteSteps == kVoteSteps - 1)
                 flush_free = __all_sync(0xffffffffu, rows_flush_free(L, dM, dI, dD));
     };
 

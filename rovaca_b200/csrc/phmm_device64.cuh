@@ -1,6 +1,5 @@
 // FP64 recompute (the pass that reruns the pairs whose FP32 sum underflowed): the lane state and step
-// of the FP32 kernels (phmm_device2.cuh) in scalar double, one read per warp, with the reference's
-// flush-to-zero.  LaneRowsEq for constant gap qualities with equal insertion and deletion quality
+// of the FP32 kernels (phmm_device2.cuh) in scalar double, one read per warp.  LaneRowsEq for constant gap qualities with equal insertion and deletion quality
 // (the FP64 classes of mode 0, PM_EQ), LaneRowsRow for per-row gap parameters (modes 1 and 2); the
 // all-FP64 check kernels keep phmm_device.cuh's sweep.
 //
@@ -8,9 +7,11 @@
 // D[i][j+1]; the lane above forms the lane's first-row I and diagonal sum from its bottom row (mm,
 // gapm and mx are one value per read), so a step shuffles two doubles.  Per cell the reference's
 // operations on the same operands as phmm_device.cuh `cells` (M * mx, formed once, is also M * my
-// since mx == my), each result flushed below 2^-1022 unless the warp's vote has shown that no result
-// of the step can fall there: the same results bit for bit, with 2 K + 3 doubles of lane state
-// instead of 4 K + 3, two shuffles instead of three, and (PM_EQ) 7 operations per cell instead of 8.
+// since mx == my), with 2 K + 3 doubles of lane state instead of 4 K + 3, two shuffles instead of three,
+// and (PM_EQ) 7 operations per cell instead of 8.  The reference flushes every result below 2^-1022 to 0.
+// Here a run is swept without flushes, and its pairs whose sum is below 2^-700 again with a flush after
+// every operation: those have the reference's bits by construction, the others as explained at
+// kUnflushedMin.
 #pragma once
 
 #include "phmm_device.cuh"
@@ -223,9 +224,11 @@ __device__ __forceinline__ double row_diag(const LaneRowsRow<K>& L, int k, doubl
 // The pass sweeps without flushes first.  A result below 2^-1022 that the reference flushes to 0 is then
 // kept, which can only matter to values near it: every operation adds products with factors of at most 1,
 // so what the flushes take away stays below about 2^-1000 in any later value, and a value of 2^-700 or
-// more, which has no bits below 2^-753, is the same with and without it (but for a sum that falls exactly
-// on a rounding tie).  A pair whose sum is below 2^-700, a likelihood below 1e-517, is swept again with the
-// reference's flush after every operation; so is one whose sum is 0.
+// more, which has no bits below 2^-753, is the same with and without it, but where a sum of larger values
+// lies exactly on a rounding tie, or within 2^-1000 of one: then its last bit may differ from the
+// reference's (one in 2^50 operations or fewer; no such pair is known).  A pair whose sum is below 2^-700, a
+// likelihood below 1e-517, is swept again with the reference's flush after every operation; so is one whose
+// sum is 0.
 // Before, every step either flushed (about three integer operations per FP64 operation, more than the
 // FP64 work itself) or ran without under a warp vote that no result could fall below 2^-1022, which long
 // reads rarely pass: far from a read's alignment there are always values around 2^-1022.  Measured on

@@ -1154,10 +1154,12 @@ struct ChunkRange {
 // Cuts a validated batch in two at the region boundary near a share of its cells: a small first chunk gets
 // the device going after little planning and uploading, and the rest is planned and uploaded while it
 // runs, so its share (5% to 25% of the cells) follows the batch's bytes per cell, kFirstCellsPerByte cells
-// per byte of the batch, and a fixed cost of kFirstCells.  Measured on B200 end to end, in ms, at 110 and
-// 200 cells per byte: 1,000 benchmark regions (8.0e-4 bytes per cell) 102.8 and 103.5, 150 regions with
-// per-base gaps (8.4e-4) 20.5 and 20.7, 1,500 regions at whole-genome depth (1.2e-3) 22.9 and 22.0, 200 of
-// them 3.6 and 3.5, 20 benchmark regions 2.55 and 2.35.  Two cuts (at 4% and 20%, 6% and 30%, 10% and 40%)
+// per byte of the batch, and a fixed cost of kFirstCells.  Measured on B200 end to end, in ms (medians of
+// three processes), at 70, 110, 130 and 200 cells per byte: 1,000 benchmark regions (8.0e-4 bytes per cell)
+// 102.4, 102.2, 102.3, 102.9; 150 regions with per-base gaps (8.4e-4) 20.3, 20.6, 20.7, 20.8; 1,500 regions
+// at whole-genome depth (1.2e-3) 23.3, 21.7, 21.6, 22.0; 600 regions of 300 reads of 100 bases 38.5, 37.4,
+// 37.3, 37.7; with a fixed part of 0, 3e8, 6e8 and 12e8 cells: 20 benchmark regions 2.29, 2.17, 2.17, 2.21,
+// 60 of them 8.09, 8.10, 8.08, 8.18, 1,500 at whole-genome depth 21.6, 21.7, 21.6, 21.7.  Two cuts (at 4% and 20%, 6% and 30%, 10% and 40%)
 // cost 1,000 regions 4-6 ms more than one at 8%.
 constexpr double kFirstCellsPerByte = 130.0, kFirstCells = 6e8;
 

@@ -24,7 +24,7 @@
 // Bound: integer ALU issue (75% of the pipe's cycles at 16 warps per SM; long-scoreboard and
 // shared-memory waits below half a cycle per issue).  Measured on B200 on 74,776 alignments (300 regions
 // of the benchmark's shape, 4.91e9 cells), device time alone: 8.53 ms with one alignment per warp in 32
-// bits, 3.10 ms here (1,583 GCUPS).
+// bits, 2.97 ms here (1,650 GCUPS).
 //
 // Trace-back.  Lanes 0-15 follow X and lanes 16-31 Y.  Each iteration the 16 lanes look at the next 16
 // cells in the direction of the state (diagonal, or along the gap) and take the whole run at once.
@@ -168,8 +168,8 @@ __device__ inline uint32_t sw16_op(uint32_t run)
 // halves hold the difference to it plus 32768; every kSw16Rebase steps all lanes move their base to their
 // first column's H.  A shuffled value is brought to the receiver's base by one add (the bases' difference,
 // exchanged at the rebasing).  Last row and column are kept as 32-bit scores.  Measured on B200, device
-// time of 2,726 haplotype-to-window alignments with the assembly parameters: 2.14 ms with one alignment
-// per warp in 32 bits, 0.91 ms here.
+// time of 2,726 haplotype-to-window alignments with the assembly parameters: 4.48 ms with one alignment
+// per warp in 32 bits (codes by haplotype row), 0.88 ms here.
 template <int K, bool REB>
 __device__ inline void sw16_pair(const SwView& v, uint32_t ix, uint32_t iy, int lane, uint8_t* scr, char* sm,
                                  uint32_t max_rows)
