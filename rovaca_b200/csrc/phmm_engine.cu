@@ -1420,32 +1420,16 @@ phmm_status Engine::check_fp64(Slot& s, const Plan& plan, double* out, std::stri
 {
     PHMM_CK(cudaSetDevice(dev_));
     cudaStream_t m = s.main;
-    // Rerun entries covering every pair: per work item and read, the item's run of haplotypes, in
-    // the FP64 class of the read's length (modes 1 and 2 only: the check kernels take any read).
-    std::vector<std::vector<RerunEntry>> per(kClasses64);
-    for (const WorkItem& it : plan.items) {
-        const RegionDesc& rg = plan.regions[it.region];
-        for (int k = 0; k < 2; ++k) {
-            const uint32_t r = it.read[k];
-            if (r == kNoRead) continue;
-            RerunEntry e;
-            e.out_idx = rg.out_off + (uint64_t)it.hap_lo * rg.n_reads + (r - rg.read_begin);
-            e.read = r;
-            e.hap = rg.hap_begin + it.hap_lo;
-            e.n_haps = (uint32_t)(it.hap_hi - it.hap_lo);
-            e.out_stride = rg.n_reads;
-            const uint64_t R = plan.read_off[r + 1] - plan.read_off[r];
-            per[class64_for_len(it.variant == kIntra ? 2 : 1, R)].push_back(e);
-        }
-    }
     std::vector<RerunEntry> all;
-    std::vector<ClassDesc> cd(kClasses64);
-    for (int c = 0; c < kClasses64; ++c) {
-        cd[c] = ClassDesc{};
-        cd[c].rerun_off = (uint32_t)all.size();
-        cd[c].rerun_cap = cd[c].rerun_count = (uint32_t)per[c].size();
-        all.insert(all.end(), per[c].begin(), per[c].end());
-    }
+    std::vector<ClassDesc> cd;
+    // sized to the batch like the work items, but for one read a warp and fewer warps, since a run's set-up
+    // costs these kernels more.  Measured on B200 with the work items' runs, and sized for 8, 4 and 2 warps
+    // per SM, in ms: 20 benchmark regions 12.2, 10.6, 10.8, 11.6, 60 of them 34.6, 30.6, 30.4, 30.8, 200 88.6,
+    // 84.1, 83.7, 83.2, 10 low-quality regions 9.05, 9.06, 8.80, 8.53.
+    uint64_t stream = 0;
+    for (const RegionDesc& rg : plan.regions)
+        stream += (plan.hap_off[rg.hap_begin + rg.n_haps] - plan.hap_off[rg.hap_begin]) * rg.n_reads;
+    all_pair_runs(plan, run_cols_for(stream, (uint64_t)sms_ * 4), all, cd);
     if (all.size() > s.cap.rerun) {
         err = "check entries exceed the slot's rerun capacity";
         return PHMM_ERR_INTERNAL;
@@ -1475,12 +1459,12 @@ phmm_status Engine::check_fp64(Slot& s, const Plan& plan, double* out, std::stri
     const uint64_t warps = scratch_warps();
     const unsigned int scr_cols = s.cap.scratch_cols ? (unsigned int)(s.cap.scratch_cols / warps) : 0u;
     for (int c = 9; c < kClasses64; ++c) {
-        if (per[c].empty()) continue;
+        if (cd[c].rerun_count == 0) continue;
         const bool multi = c % 9 == 8;
         const int region = 1 + c / 9;
         int occ = 0;
         PHMM_CK(occupancy_f64_check(c, &occ));
-        uint64_t grid = std::min<uint64_t>(per[c].size(), (uint64_t)std::max(occ, 1) * sms_);
+        uint64_t grid = std::min<uint64_t>(cd[c].rerun_count, (uint64_t)std::max(occ, 1) * sms_);
         if (multi) grid = std::min(grid, scratch_offset_warps(region + 1) - scratch_offset_warps(region));
         PassControl pc{};
         pc.cd = s.d_classes + kClasses32 + c;

@@ -455,4 +455,48 @@ phmm_status build_plan(const phmm_batch& b, const PlanLimits& lim, Plan& plan, s
     return PHMM_OK;
 }
 
+void all_pair_runs(const Plan& plan, uint32_t max_cols, std::vector<RerunEntry>& all, std::vector<ClassDesc>& cd)
+{
+    constexpr uint32_t kBuckets = 64, kBucketCols = 128;
+    const uint32_t single = std::min(PlanLimits().max_stream_single, max_cols);
+    const uint32_t striped = std::min(PlanLimits().max_stream_multi, std::max(max_cols / 2, 1u));
+    std::vector<std::vector<RerunEntry>> per((size_t)kClasses64 * kBuckets);
+    std::vector<Run> runs[4];  // for single- and multi-stripe reads without and with an N
+    for (uint32_t g = 0; g < plan.n_regions; ++g) {
+        const RegionDesc& rg = plan.regions[g];
+        const uint64_t* hoff = plan.hap_off.data() + rg.hap_begin;
+        for (auto& r : runs) r.clear();
+        for (uint32_t q = 0; q < rg.n_reads; ++q) {
+            const uint32_t r = rg.read_begin + q;
+            const uint64_t R = plan.read_off[r + 1] - plan.read_off[r];
+            if (R == 0) continue;
+            const bool read_n = (plan.read_flags[r] & 1) != 0, multi = R > (uint64_t)kWarp * kMaxK;
+            std::vector<Run>& rr = runs[(multi ? 2 : 0) + (read_n ? 1 : 0)];
+            if (rr.empty())
+                make_runs(hoff, plan.hap_flags.data() + rg.hap_begin, rg.n_haps,
+                          multi ? striped : single, !read_n, rr);
+            for (const Run& run : rr) {
+                RerunEntry e;
+                e.out_idx = rg.out_off + (uint64_t)run.lo * rg.n_reads + q;
+                e.read = r;
+                e.hap = rg.hap_begin + run.lo;
+                e.n_haps = (uint32_t)(run.hi - run.lo);
+                e.out_stride = rg.n_reads;
+                const int c = class64_for_len(run.variant == kIntra ? 2 : 1, R);
+                per[(size_t)c * kBuckets + kBuckets - 1 - std::min(run.cols / kBucketCols, kBuckets - 1)].push_back(e);
+            }
+        }
+    }
+    all.clear();
+    cd.assign(kClasses64, ClassDesc{});
+    for (int c = 0; c < kClasses64; ++c) {
+        cd[c].rerun_off = (uint32_t)all.size();
+        for (uint32_t b = 0; b < kBuckets; ++b) {
+            const auto& v = per[(size_t)c * kBuckets + b];
+            all.insert(all.end(), v.begin(), v.end());
+        }
+        cd[c].rerun_cap = cd[c].rerun_count = (uint32_t)all.size() - cd[c].rerun_off;
+    }
+}
+
 }  // namespace phmm

@@ -112,4 +112,10 @@ phmm_status scan_batch(const phmm_batch& b, const PlanLimits& lim, BatchScan& s,
 // scan_batch, then the full plan.  Same return codes.
 phmm_status build_plan(const phmm_batch& b, const PlanLimits& lim, Plan& plan, std::string& err);
 
+// Runs covering every pair of a planned batch in the FP64 classes of modes 1 and 2 (whose check kernels take
+// any read), of at most max_cols columns where a haplotype is not longer (half of that for multi-stripe
+// reads), longest first in a class; cd receives the classes' segments of `all`.  There are no more of them
+// than pairs.
+void all_pair_runs(const Plan& plan, uint32_t max_cols, std::vector<RerunEntry>& all, std::vector<ClassDesc>& cd);
+
 }  // namespace phmm

@@ -2,7 +2,8 @@
 //   plan_check cover SEED   random regions, with empty sequences, N, long reads and short runs: every pair of a
 //                           non-empty read and haplotype is in exactly one work item, the items of a class
 //                           lie together, longest streams first and regions in order within 128 columns, and
-//                           the class and rerun counts add up
+//                           the class and rerun counts add up; the runs of the all-FP64 check cover every
+//                           pair once too, in no more runs than the longest streams need
 //   plan_check cost         planning time of one batch cut into one item per read pair and into one per read
 //                           pair and haplotype (best of 40, microseconds)
 #include <algorithm>
@@ -95,6 +96,38 @@ int cover(int seed)
                 if (seen[rg.out_off + (uint64_t)h * rg.n_reads + r] != full) return 6;
             }
     }
+    std::vector<RerunEntry> all;
+    std::vector<ClassDesc> cd;
+    all_pair_runs(p, 8192, all, cd);
+    std::vector<uint8_t> again(p.out_total, 0);
+    uint64_t least = 0;
+    for (uint32_t g = 0; g < p.n_regions; ++g) {  // every region fits one stream per N-free stretch here
+        const RegionDesc& rg = p.regions[g];
+        uint64_t groups = 0;
+        int last = -1;
+        for (uint32_t h = rg.hap_begin; h < rg.hap_begin + rg.n_haps; ++h) {
+            const int kind = p.hap_off[h + 1] == p.hap_off[h] ? -1 : p.hap_flags[h] & 1;
+            groups += kind >= 0 && kind != last;
+            last = kind;
+        }
+        least += groups * rg.n_reads;
+    }
+    if (all.size() > least) return 8;
+    for (int c = 0; c < kClasses64; ++c) {
+        uint64_t bucket = ~0ull;
+        for (uint32_t k = cd[c].rerun_off; k < cd[c].rerun_off + cd[c].rerun_count; ++k) {
+            const RerunEntry& e = all[k];
+            const uint64_t R = p.read_off[e.read + 1] - p.read_off[e.read];
+            const bool n = (p.read_flags[e.read] | p.hap_flags[e.hap]) & 1;
+            if (c != class64_for_len(n ? 2 : 1, R)) return 9;
+            const uint64_t bk = std::min<uint64_t>((p.hap_off[e.hap + e.n_haps] - p.hap_off[e.hap]) / 128, 63);
+            if (bk > bucket) return 10;
+            bucket = bk;
+            for (uint32_t h = 0; h < e.n_haps; ++h)
+                if (again[e.out_idx + (uint64_t)h * e.out_stride]++) return 11;
+        }
+    }
+    if (again != seen) return 12;
     return pairs == p.pairs && cells == p.cells && rerun == pairs && p.empty_pairs == p.out_total - pairs ? 0 : 7;
 }
 
