@@ -164,15 +164,19 @@ PHMM_HD inline Sw16Layout sw16_layout(uint32_t max_rows, int K)
 template <typename Col>
 uint64_t realign_scratch_bytes(uint32_t rows, uint32_t n, Col col)
 {
-    uint32_t count[kSwWrapClass] = {};
+    constexpr uint32_t kWidest = kSwK[kSwWrapClass - 1];
+    uint32_t count[kWidest + 1] = {};  // by width in 32 columns
     for (uint32_t q = 0; q < n; ++q) {
-        int c = 0;
-        while (c + 1 < kSwWrapClass && 32u * (uint32_t)kSwK[c] < col(q)) ++c;
-        ++count[c];
+        const uint32_t w = (col(q) + 31) / 32;
+        ++count[w < kWidest ? w : kWidest];
     }
     uint64_t bytes = 0;
-    for (int c = 0; c < kSwWrapClass; ++c)
-        if (count[c]) bytes += ((uint64_t)count[c] + 1) / 2 * sw16_layout(rows, kSwK[c]).total;
+    uint32_t w = 0;
+    for (int c = 0; c < kSwWrapClass; ++c) {
+        uint64_t of_class = 0;
+        for (; w <= (uint32_t)kSwK[c]; ++w) of_class += count[w];
+        if (of_class) bytes += (of_class + 1) / 2 * sw16_layout(rows, kSwK[c]).total;
+    }
     return bytes;
 }
 
